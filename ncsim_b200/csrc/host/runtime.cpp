@@ -18,8 +18,6 @@ PolyTerms build_poly_terms(const PhasePolyIR& p, const std::vector<uint32_t>& qu
 struct PlainPlan;
 std::shared_ptr<PlainPlan> plan_plain_passes(uint32_t n, int precision, const std::vector<const LoweredOp*>& gates);
 void run_plain_plan(ncsim_state* s, PlainPlan& P);
-size_t plain_plan_passes(const PlainPlan& P);
-size_t plain_plan_pass_gates(const PlainPlan& P);
 
 void apply_lowered(ncsim_state* s, const LoweredOp& op) {
   switch (op.kind) {

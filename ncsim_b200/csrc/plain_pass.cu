@@ -1,12 +1,13 @@
 // Tiled passes of the plain path: a run of consecutive gates applied to tiles
 // of the register in shared memory, one read and one write of HBM for the run.
 //
-// A pass picks a window of T <= 12 qubits (the qubits the run's gates move,
+// A pass picks a window of T <= 11 qubits (the qubits the run's gates move,
 // filled up with the lowest other qubits so that tiles load in runs of
 // consecutive amplitudes) and streams the register's 2^(n-T) tiles through
 // shared memory: a persistent CTA double-buffers its tiles (cp.async copies
 // of the next tile land while the current one is worked on) and applies the
-// pass's gates to each tile in circuit order, one __syncthreads between gates.
+// pass's gates to each tile in circuit order, in chains of gates that work on
+// amplitudes held in registers, one __syncthreads between chains.
 // Gates that only multiply amplitudes by phases (diagonals, phase polynomials)
 // join any pass: their phases depend on index bits outside the window only
 // through the tile's base index.
@@ -14,9 +15,15 @@
 // Every gate is applied with the arithmetic of the kernel that the gate-by-gate
 // path would launch for it (the same dispatch rules, the same cmul/cfma
 // expressions on the same operands in the same order), so a run gives the same
-// amplitudes either way.  Gates with no tile form (dense gates on more than 3
+// amplitudes either way.  Gates with no tile form (dense gates on two or more
 // qubits, permutation tables other than pair swaps, phase polynomials of more
-// than 64 terms) run as their own kernels between passes.
+// than MAX_PASS_TERMS terms) run as their own kernels between passes.
+//
+// What bounds a pass: instruction issue and its latency (random layers at n = 24,
+// ncu: issue slots 47% busy, FP64 pipe 27%, shared memory 29%, DRAM 18%), not HBM.
+// Measured on random layers of depth 20, complex128, against 8-amplitude cubes on
+// 4096-amplitude tiles (one 512-thread CTA per SM): n = 20 0.80 -> 0.49 ms, n = 24
+// 11.8 -> 5.3 ms, n = 28 221 -> 100 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -31,49 +38,115 @@ namespace ncsim {
 
 namespace {
 
-constexpr int PASS_THREADS = 512;
-constexpr int MAX_TILE_BITS = 12;
-constexpr int MAX_FIBER_K = 3;  // 4- and 5-qubit matrices run as their own kernels (registers)
+// Tiles of 2^11 amplitudes: 128 threads with 16 amplitudes each, 64 KB for two complex128
+// buffers, three CTAs per SM that drift apart and so overlap one's loads and barriers with
+// another's arithmetic.  Tiles of 2^12 (one CTA of 256 threads per SM) take fewer passes but
+// run slower (n = 28: 132 ms against 100 ms), tiles of 2^10 take more passes (n = 28: +15%).
+constexpr int MAX_TILE_BITS = 11;
+// On registers of more than this many qubits a window always holds the two lowest qubits,
+// so that a tile is read and written in runs of 64 bytes (complex128).  A window of high
+// qubits alone touches single amplitudes: one pass at n = 26 took 1.79 ms against 0.83 ms.
+// Smaller registers stay in the L2 and lose more by the extra passes (n = 16: 10 against 8).
+constexpr int FREE_WINDOW_QUBITS = 18;
+constexpr int LOW_WINDOW_BITS = 2;
 constexpr int MAX_TABLE_K = 10;
 // longer phase polynomials run as the bit-sliced kernel: evaluated per element
 // in a tile they cost a popcount per parity per amplitude
 constexpr int MAX_PASS_TERMS = 4;
 constexpr int MAX_PASS_PARITIES = 8;
-constexpr int MAX_PASS_OPS = 192;  // ops of one pass (chain heads included)
+constexpr int MAX_PASS_OPS = 240;  // device ops of one pass (chain heads and flushes included)
+constexpr int MAX_PASS_CHAINS = MAX_PASS_OPS / 3;
+// A chain's cube: CUBE_BITS tile bits, CUBE amplitudes held by one thread.  Four
+// bits: the op fetch and dispatch (about 25 instructions) are shared by 16
+// amplitudes, and a layer's 12 window qubits need 3 to 4 shared-memory round
+// trips.  The earlier three-bit cubes on 512 threads spent 54% of all issue slots
+// with the FP64 pipe 23% busy.
+constexpr int CUBE_BITS = 4;
+constexpr int CUBE = 1 << CUBE_BITS;
 
 template <class R>
 using V = typename VecOf<R>::T;
 
 enum TileKind : uint32_t {
   TK_DENSE1,      // 1-qubit dense matrix (k_dense1)
-  TK_DENSE2,      // 2-qubit dense matrix (k_dense2)
-  TK_FIBER,       // 3-qubit dense matrix (k_dense_fiber)
   TK_DIAG_CONST,  // one phase on the indices with every fixed bit set (k_diag_const)
   TK_DIAG_1Q,     // two phases selected by one bit (k_diag_1q)
   TK_DIAG_TABLE,  // phase table over <= 10 qubits (k_diag)
   TK_PAIRSWAP,    // exchange of i and i ^ x on a fixed-bit sub-cube (k_pairswap)
   TK_PHASEPOLY,   // phase polynomial of the global index (k_phasepoly)
-  TK_CHAIN,       // the next k ops, applied group by group to 8-element cubes held in registers
 };
+
+// What the device executes.  Inside a chain the element of a cube that an op
+// touches is known when the chain is made, so the common ops come in one kind
+// per cube bit, with register indices fixed at compile time.
+enum DevKind : uint32_t {
+  DK_CHAIN = 0,                      // the next k ops, on cubes held in registers
+  DK_D1 = 1,                         // + j: dense 2x2 on cube bit j
+  DK_D1R = DK_D1 + CUBE_BITS,        // + j: a real matrix (RY): the zero products left out
+  DK_D1RE = DK_D1R + CUBE_BITS,      // + j: a real matrix with equal entries in its first column (H): one product for both
+  DK_D1X = DK_D1RE + CUBE_BITS,      // + j: real diagonal, imaginary off-diagonal (RX)
+  DK_D1E = DK_D1X + CUBE_BITS,       // + j: equal entries in the first column (SQRT_Y)
+  DK_D1S = DK_D1E + CUBE_BITS,       // + j: first column (1+i)/2, (1-i)/2 (SQRT_X)
+  DK_D1SD = DK_D1S + CUBE_BITS,      // + j: first column (1-i)/2, (1+i)/2 (SQRT_X_DAG)
+  DK_PH = DK_D1SD + CUBE_BITS,        // + j: phase on the half of the cube with bit j set
+  DK_PH_ALL = DK_PH + CUBE_BITS,     // phase on the whole cube
+  DK_PH_MASK,                        // phase on the cube elements of a mask
+  DK_TURN,                           // + j: quarter turn (+-i) on the half with bit j set: parts exchanged, one negated
+  DK_TURN_ALL = DK_TURN + CUBE_BITS,
+  DK_TURN_MASK,
+  DK_SIGN,                           // sign of the cube elements of a mask, kept pending in a bit mask
+  DK_FLUSH,                          // the pending signs applied
+  DK_RZ,                             // + j: two phases selected by cube bit j
+  DK_RZ_OUT = DK_RZ + CUBE_BITS,     // two phases selected by a tile bit outside the cube
+  DK_SWAP,                           // + index of the xor mask: exchange inside the cube (no phases)
+  DK_SWAPC = DK_SWAP + 10,           // + index of the xor mask: exchange with phases
+  DK_TABLE = DK_SWAPC + 10,          // phase table
+  DK_POLY,                           // phase polynomial
+  DK_TILE_SWAP,                      // exchange across more than two tile bits: its own sweep over the tile
+  DK_COND = 0x8000,                  // set when the op has fixed bits outside the window (gfix, gval)
+};
+// the xor masks of an exchange on one or two cube bits, in DK_SWAP's order
+constexpr uint32_t SWAP_X[10] = {1, 2, 4, 8, 3, 5, 9, 6, 10, 12};
 
 // One gate of a pass, encoded against the pass's window: "local" masks are
 // over the tile's T bits, "global" masks over the bits outside the window.
 struct TileOp {
   uint32_t kind;
-  uint32_t k;        // qubits (fiber, table), terms (phase polynomial)
-  uint32_t l0, l1;   // local bit positions (dense1: l0; dense2: l0 = qubit 0, l1 = qubit 1; diag 1q: l1 = global qubit outside)
+  uint32_t k;        // qubits (table), terms (phase polynomial)
+  uint32_t l0, l1;   // local bit positions (dense1: l0; diag 1q: l0, or l1 = the global qubit outside)
   uint32_t lfix;     // local mask of fixed bits
   uint32_t lones;    // the fixed bits' values at i (pairswap), or lfix (diagonal kinds)
   uint32_t lx;       // local xor mask (pairswap)
-  uint32_t flags;    // pairswap: unit_i | unit_j << 1; diag 1q: 1 = the qubit lies outside (value in gval)
+  uint32_t flags;    // pairswap: unit_i | unit_j << 1; diag 1q: 1 = the qubit lies outside
   uint64_t gfix;     // fixed bits outside the window ...
   uint64_t gval;     // ... and the values the tile base must have there
   uint64_t gz;       // phase polynomial: offset of its parities
-  uint32_t phase;
   uint32_t cp;       // complex pool offset
   uint32_t up;       // word pool offset
-  uint32_t reg;      // in a chain: the op's bits among the cube's three, or its cube elements (see chainify)
-  uint32_t gml, gvl; // in a chain: fixed local bits outside the cube, and their values
+};
+
+// One device op.  Its head (what it is and what selects its elements) stays in the
+// kernel parameters, where a warp reads it into uniform registers: the op loop's
+// branches are then uniform ones.  The constants are read from shared memory.
+struct OpHead {
+  uint32_t kind;
+  uint32_t em;        // cube elements (bit b: element b); chain: number of ops
+  uint32_t gml, gvl;  // fixed tile bits outside the cube, and their values; chain: cube bits, chain number
+};
+struct OpCond {
+  uint64_t gfix, gval;  // fixed bits outside the window, and the values the tile base must have there
+};
+template <class R>
+struct alignas(16) OpArgs {
+  union {
+    V<R> c[4];
+    uint32_t a[8];    // table: k, lfix, lones, up, cp; polynomial: k, up, cp, parity offset; tile swap: see tile_pairswap;
+  };                  // chain: the tile bits of the thread's index, one byte each, in a[0], a[1]
+};
+struct DevOp {
+  OpHead h{};
+  OpCond g{};
+  OpArgs<double> x{};
 };
 
 struct PassGeom {
@@ -107,21 +180,28 @@ __device__ __forceinline__ uint32_t insert_zeros32(uint32_t v, const uint8_t* po
   }
   return v;
 }
-__device__ __forceinline__ int parity64(uint64_t v) { return __popcll(v) & 1; }
 
-// A tile in shared memory, element e stored at e ^ ((e >> 3) & 7): the XOR of
-// the low three index bits with the next three spreads the 16-byte elements of
-// a warp's access over the banks whichever tile bits an op pairs (a thread
-// holding a cube of three low bits reads eight consecutive elements; without
-// the swizzle every thread of the warp would hit the same four banks).
+// A tile in shared memory: element e at e ^ (the XOR of e's higher groups of SB
+// bits), SB = 3 for 16-byte elements and 4 for 8-byte ones, so tile bit b moves
+// the bank group by bit b mod SB.  Lanes whose lowest SB bits sit on tile bits of
+// distinct residues mod SB hit distinct banks; chain heads order their thread bits
+// that way.  The map is linear over XOR: a thread's and an element's part combine.
+template <class R>
+__host__ __device__ __forceinline__ uint32_t swz(uint32_t e) {
+  if constexpr (sizeof(V<R>) == 16) return e ^ (((e >> 3) ^ (e >> 6) ^ (e >> 9)) & 7u);
+  else return e ^ (((e >> 4) ^ (e >> 8)) & 15u);
+}
+template <class R>
+__device__ __forceinline__ V<R>* shared_tile() {
+  extern __shared__ __align__(16) unsigned char pass_smem[];
+  return reinterpret_cast<V<R>*>(pass_smem);
+}
 template <class R>
 struct SwTile {
   V<R>* p;
-  __device__ __forceinline__ V<R>& operator[](uint32_t e) const { return p[e ^ ((e >> 3) & 7u)]; }
+  __device__ __forceinline__ V<R>& operator[](uint32_t e) const { return p[swz<R>(e)]; }
 };
 
-// The pass's ops travel in the kernel parameters (constant bank): every thread
-// reads the same op at the same time, a broadcast the constant cache serves.
 template <class R>
 struct PassParams {
   V<R>* amp;
@@ -131,143 +211,29 @@ struct PassParams {
   const V<R>* cpool;
   const uint32_t* upool;
   const uint64_t* ppool;  // phase polynomial parities (global masks)
-  TileOp ops[MAX_PASS_OPS];
+  uint32_t nchains;
+  OpHead head[MAX_PASS_OPS];
+  OpCond cond[MAX_PASS_OPS];
+  OpArgs<R> args[MAX_PASS_OPS];  // copied into shared memory once per CTA
 };
 
-// constant i of the pass's pool
-template <class R>
-__device__ __forceinline__ V<R> pconst(const PassParams<R>& P, uint32_t i) {
-  return P.cpool[i];
+// x with its sign bit xored by s (0 or 0x80000000)
+__device__ __forceinline__ double flip(double x, uint32_t s) {
+  return __hiloint2double(int(uint32_t(__double2hiint(x)) ^ s), __double2loint(x));
 }
+__device__ __forceinline__ float flip(float x, uint32_t s) { return __uint_as_float(__float_as_uint(x) ^ s); }
 
-// -------- the gates on a tile (all threads of the CTA; `t` in shared memory) --------
+// exchange across three or more tile bits: a: number of fixed bits, their positions in the word pool, pairswap flags, xor mask, values
 template <class R>
-__device__ void tile_dense1(SwTile<R> t, uint32_t tsz, const TileOp& op, const V<R>* cp) {
-  const V<R> m00 = cp[op.cp], m01 = cp[op.cp + 1], m10 = cp[op.cp + 2], m11 = cp[op.cp + 3];
-  const uint32_t lo = (1u << op.l0) - 1;
-  for (uint32_t p = threadIdx.x; p < (tsz >> 1); p += blockDim.x) {
-    const uint32_t i0 = ((p & ~lo) << 1) | (p & lo), i1 = i0 | (lo + 1);
-    const V<R> a0 = t[i0], a1 = t[i1];
-    t[i0] = cfma(m01, a1, cmul(m00, a0));
-    t[i1] = cfma(m11, a1, cmul(m10, a0));
-  }
-}
-
-template <class R>
-__device__ void tile_dense2(SwTile<R> t, uint32_t tsz, const TileOp& op, const V<R>* cp) {
-  const uint32_t ba = 1u << op.l0, bb = 1u << op.l1;
-  uint8_t pos[2] = {uint8_t(min(op.l0, op.l1)), uint8_t(max(op.l0, op.l1))};
-  for (uint32_t p = threadIdx.x; p < (tsz >> 2); p += blockDim.x) {
-    const uint32_t i = insert_zeros32(p, pos, 2);
-    const uint32_t idx[4] = {i, i | ba, i | bb, i | ba | bb};
-    V<R> v[4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) v[b] = t[idx[b]];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      V<R> acc = cmul(cp[op.cp + 4 * r], v[0]);
-      acc = cfma(cp[op.cp + 4 * r + 1], v[1], acc);
-      acc = cfma(cp[op.cp + 4 * r + 2], v[2], acc);
-      acc = cfma(cp[op.cp + 4 * r + 3], v[3], acc);
-      t[idx[r]] = acc;
-    }
-  }
-}
-
-template <class R, int K>
-__device__ void tile_fiber(SwTile<R> t, uint32_t tsz, const TileOp& op, const V<R>* cp, const uint32_t* up) {
-  constexpr int D = 1 << K;
-  uint8_t pos[K];
-#pragma unroll
-  for (int j = 0; j < K; ++j) pos[j] = uint8_t(up[op.up + j]);
-  uint32_t off[D];
-#pragma unroll
-  for (int b = 0; b < D; ++b) off[b] = up[op.up + K + b];
-  const V<R>* m = cp + op.cp;
-  for (uint32_t f = threadIdx.x; f < (tsz >> K); f += blockDim.x) {
-    const uint32_t base = insert_zeros32(f, pos, K);
-    V<R> v[D];
-#pragma unroll
-    for (int b = 0; b < D; ++b) v[b] = t[base | off[b]];
-#pragma unroll
-    for (int r = 0; r < D; ++r) {
-      V<R> acc = cmul(m[r * D], v[0]);
-#pragma unroll
-      for (int b = 1; b < D; ++b) acc = cfma(m[r * D + b], v[b], acc);
-      t[base | off[r]] = acc;
-    }
-  }
-}
-
-// the elements with every local fixed bit set to its value: p with zeros inserted, ORed with the values
-template <class R>
-__device__ void tile_diag_const(SwTile<R> t, uint32_t tsz, const TileOp& op, const V<R>* cp, const uint32_t* up) {
-  const int nf = __popc(op.lfix);
+__device__ void tile_pairswap(SwTile<R> t, uint32_t tsz, const OpArgs<R>& op, const V<R>* cpool, const uint32_t* up) {
+  const int nf = int(op.a[0]);
   uint8_t pos[MAX_TILE_BITS];
-  for (int i = 0; i < nf; ++i) pos[i] = uint8_t(up[op.up + i]);
-  const V<R> c = cp[op.cp];
+  for (int i = 0; i < nf; ++i) pos[i] = uint8_t(up[op.a[1] + i]);
+  const bool ui = op.a[2] & 1, uj = (op.a[2] >> 1) & 1;
+  const V<R> ci = cpool[op.a[5]], cj = cpool[op.a[5] + 1];
   for (uint32_t p = threadIdx.x; p < (tsz >> nf); p += blockDim.x) {
-    const uint32_t e = insert_zeros32(p, pos, nf) | op.lones;
-    const V<R> u = t[e];
-    if (!is_zero(u)) t[e] = cmul(c, u);
-  }
-}
-
-template <class R>
-__device__ void tile_diag_1q(SwTile<R> t, uint32_t tsz, const TileOp& op, const V<R>* cp, uint64_t base) {
-  const V<R> c0 = cp[op.cp], c1 = cp[op.cp + 1];
-  const bool outside = op.flags & 1;
-  const bool obit = (base >> op.l1) & 1;  // the qubit's global position when it lies outside
-  for (uint32_t e = threadIdx.x; e < tsz; e += blockDim.x) {
-    const V<R> u = t[e];
-    const bool bit = outside ? obit : ((e >> op.l0) & 1u);
-    if (!is_zero(u)) t[e] = cmul(bit ? c1 : c0, u);
-  }
-}
-
-template <class R>
-__device__ void tile_diag_table(SwTile<R> t, uint32_t tsz, const TileOp& op, const V<R>* cp, const uint32_t* up,
-                                uint64_t base) {
-  // up: [k] local position of qubit j (or 255 + its global position when outside), then the
-  // local fixed positions (ascending), then the unit flags as bytes
-  const int k = int(op.k);
-  const int nf = __popc(op.lfix);
-  uint32_t xout = 0;
-  uint8_t lpos[MAX_TABLE_K];
-  for (int j = 0; j < k; ++j) {
-    const uint32_t v = up[op.up + j];
-    if (v >= 256) {
-      xout |= uint32_t((base >> (v - 256)) & 1u) << j;
-      lpos[j] = 255;
-    } else {
-      lpos[j] = uint8_t(v);
-    }
-  }
-  uint8_t fpos[MAX_TILE_BITS];
-  for (int i = 0; i < nf; ++i) fpos[i] = uint8_t(up[op.up + k + i]);
-  const uint8_t* unit = reinterpret_cast<const uint8_t*>(up + op.up + k + nf);
-  const V<R>* d = cp + op.cp;
-  for (uint32_t p = threadIdx.x; p < (tsz >> nf); p += blockDim.x) {
-    const uint32_t e = insert_zeros32(p, fpos, nf) | op.lones;
-    uint32_t x = xout;
-    for (int j = 0; j < k; ++j)
-      if (lpos[j] != 255) x |= ((e >> lpos[j]) & 1u) << j;
-    if (unit[x]) continue;
-    const V<R> v = t[e];
-    if (!is_zero(v)) t[e] = cmul(d[x], v);
-  }
-}
-
-template <class R>
-__device__ void tile_pairswap(SwTile<R> t, uint32_t tsz, const TileOp& op, const V<R>* cp, const uint32_t* up) {
-  const int nf = __popc(op.lfix);
-  uint8_t pos[MAX_TILE_BITS];
-  for (int i = 0; i < nf; ++i) pos[i] = uint8_t(up[op.up + i]);
-  const V<R> ci = cp[op.cp], cj = cp[op.cp + 1];
-  const bool ui = op.flags & 1, uj = (op.flags >> 1) & 1;
-  for (uint32_t p = threadIdx.x; p < (tsz >> nf); p += blockDim.x) {
-    const uint32_t i = insert_zeros32(p, pos, nf) | op.lones;
-    const uint32_t j = i ^ op.lx;
+    const uint32_t i = insert_zeros32(p, pos, nf) | op.a[4];
+    const uint32_t j = i ^ op.a[3];
     const V<R> vi = t[i], vj = t[j];
     t[i] = ui ? vj : cmul(ci, vj);
     t[j] = uj ? vi : cmul(cj, vi);
@@ -299,311 +265,407 @@ __device__ __forceinline__ double2 pass_root(uint64_t f, uint32_t bits) {
   return make_double2(c, s);
 }
 
-// up: bits, use_table, scalar_is_one, constant lo, constant hi, start[k+1], coeff[k]; cp: scalar, table[2^bits]
-template <class R>
-__device__ void tile_phasepoly(SwTile<R> t, uint32_t tsz, const TileOp& op, const V<R>* cp, const uint32_t* up,
-                               const uint64_t* pp, uint64_t base, uint64_t dthread, const uint64_t* dround) {
-  const uint32_t* u = up + op.up;
-  const uint32_t bits = u[0];
-  const bool use_table = u[1], s_one = u[2];
-  const uint64_t constant = uint64_t(u[3]) | (uint64_t(u[4]) << 32);
-  const int nt = int(op.k);
-  const uint32_t* start = u + 5;
-  const uint32_t* coeff = start + nt + 1;
-  const uint64_t modmask = (uint64_t(1) << bits) - 1;
-  const V<R> scalar = cp[op.cp];
-  const V<R>* table = cp + op.cp + 1;
-  const uint32_t nr = tsz / blockDim.x;
-  for (uint32_t r = 0; r < max(nr, 1u); ++r) {
-    const uint32_t e = threadIdx.x + r * blockDim.x;
-    if (e >= tsz) break;
-    const uint64_t i = base | dthread | dround[r];
-    const V<R> v = t[e];
-    if (is_zero(v)) continue;
-    uint64_t f = constant;
-    for (int tt = 0; tt < nt; ++tt) {
-      int all = 1;
-      for (uint32_t l = start[tt]; l < start[tt + 1]; ++l) all &= __popcll(pp[op.gz + l] & i) & 1;
-      if (all) f += coeff[tt];
-    }
-    f &= modmask;
-    V<R> c;
-    if (use_table) {
-      c = table[f];
-      if (is_one_v(c)) continue;
-    } else {
-      if (f == 0 && s_one) continue;
-      const double2 rr = pass_root(f, bits);
-      c.x = R(rr.x);
-      c.y = R(rr.y);
-      if (!s_one) c = cmul(scalar, c);
-    }
-    t[e] = cmul(c, v);
-  }
-}
-
-// ---- chains: consecutive ops whose bits lie in one cube of three tile bits ----
-// A thread holds the 8 elements of a cube (v[b]: cube pattern b) and applies
+// ---- chains: consecutive ops whose coupled bits lie in one cube of CUBE_BITS tile bits ----
+// A thread holds the elements of a cube (v[b]: cube pattern b) and applies
 // the chain's ops in order to them, one shared-memory round trip for the
 // chain.  The ops couple elements only inside a cube, and each element sees
-// its ops in circuit order with each op's own arithmetic.  Register indices
-// are compile-time: the op's cube bits (`reg`) select a template instance.
+// its ops in circuit order with each op's own arithmetic.  What gives the same
+// bits on finite amplitudes more cheaply is used: products with exact zeros are
+// left out (real matrices), +-i exchanges the parts, and -1 is a sign flip, which
+// commutes with every rounding and so waits in a mask until an op mixes elements.
+// The updates are written so that each result can take the place of an operand
+// that has just been read for the last time (both products with a0 first): the
+// cases of the op loop then meet on the same registers without copies between.
 template <class R, int J>
-__device__ __forceinline__ void chain_dense1(V<R> (&v)[8], const V<R> (&m)[4]) {
+__device__ __forceinline__ void chain_dense1(V<R> (&v)[CUBE], const V<R>* m) {
   const V<R> m00 = m[0], m01 = m[1], m10 = m[2], m11 = m[3];
 #pragma unroll
-  for (int b = 0; b < 8; ++b)
+  for (int b = 0; b < CUBE; ++b)
     if (!((b >> J) & 1)) {
-      const V<R> a0 = v[b], a1 = v[b | (1 << J)];
-      v[b] = cfma(m01, a1, cmul(m00, a0));
-      v[b | (1 << J)] = cfma(m11, a1, cmul(m10, a0));
+      V<R>&a0 = v[b], &a1 = v[b | (1 << J)];
+      V<R> p0 = cmul(m00, a0), p1 = cmul(m10, a0);  // cfma(m01, a1, p0) and cfma(m11, a1, p1):
+      p0.x = fma_rn(-m01.y, a1.y, p0.x);
+      p0.y = fma_rn(m01.y, a1.x, p0.y);
+      a0.x = fma_rn(m01.x, a1.x, p0.x);
+      a0.y = fma_rn(m01.x, a1.y, p0.y);
+      p1.x = fma_rn(-m11.y, a1.y, p1.x);
+      p1.y = fma_rn(m11.y, a1.x, p1.y);
+      a1.x = fma_rn(m11.x, a1.x, p1.x);
+      a1.y = fma_rn(m11.x, a1.y, p1.y);
     }
 }
-
-template <class R, int JA, int JB>
-__device__ __forceinline__ void chain_dense2(V<R> (&v)[8], const PassParams<R>& P, uint32_t c0) {
-  V<R> m[16];
+// A first column (1+i)/2, (1-i)/2 (S = 0), its conjugate (S = 1) or two equal entries
+// (S = 2): a product with one half is exact, so the second product is the first turned
+// by a quarter (or the same), and four of the sixteen steps go.
+template <class R, int J, int S>
+__device__ __forceinline__ void chain_dense1_col(V<R> (&v)[CUBE], const V<R>* m) {
+  const V<R> m00 = m[0], m01 = m[1], m11 = m[3];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) m[i] = pconst(P, c0 + i);
-#pragma unroll
-  for (int b = 0; b < 8; ++b)
-    if (!((b >> JA) & 1) && !((b >> JB) & 1)) {
-      const int idx[4] = {b, b | (1 << JA), b | (1 << JB), b | (1 << JA) | (1 << JB)};
-      V<R> x[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) x[q] = v[idx[q]];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        V<R> acc = cmul(m[4 * r], x[0]);
-        acc = cfma(m[4 * r + 1], x[1], acc);
-        acc = cfma(m[4 * r + 2], x[2], acc);
-        acc = cfma(m[4 * r + 3], x[3], acc);
-        v[idx[r]] = acc;
-      }
+  for (int b = 0; b < CUBE; ++b)
+    if (!((b >> J) & 1)) {
+      V<R>&a0 = v[b], &a1 = v[b | (1 << J)];
+      const V<R> p0 = cmul(m00, a0);
+      V<R> p1;
+      p1.x = S == 0 ? p0.y : S == 1 ? -p0.y : p0.x;
+      p1.y = S == 0 ? -p0.x : S == 1 ? p0.x : p0.y;
+      a0.x = fma_rn(-m01.y, a1.y, p0.x);
+      a0.y = fma_rn(m01.y, a1.x, p0.y);
+      a0.x = fma_rn(m01.x, a1.x, a0.x);
+      a0.y = fma_rn(m01.x, a1.y, a0.y);
+      p1.x = fma_rn(-m11.y, a1.y, p1.x);
+      p1.y = fma_rn(m11.y, a1.x, p1.y);
+      a1.x = fma_rn(m11.x, a1.x, p1.x);
+      a1.y = fma_rn(m11.x, a1.y, p1.y);
     }
 }
-
-// a 3-qubit matrix whose qubit j sits on cube bit PJ (the permutation P0 P1 P2)
-template <class R, int P0, int P1, int P2>
-__device__ __forceinline__ void chain_fiber(V<R> (&v)[8], const PassParams<R>& P, uint32_t c0) {
-  const V<R>* m = P.cpool + c0;
-  auto mat = [&](int i) { return m[i]; };
-  V<R> x[8];
+template <class R, int J>
+__device__ __forceinline__ void chain_dense1_real(V<R> (&v)[CUBE], const V<R>* m) {
+  const R m00 = m[0].x, m01 = m[1].x, m10 = m[2].x, m11 = m[3].x;
 #pragma unroll
-  for (int b = 0; b < 8; ++b) x[b] = v[((b & 1) << P0) | (((b >> 1) & 1) << P1) | (((b >> 2) & 1) << P2)];
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    V<R> acc = cmul(mat(r * 8), x[0]);
-#pragma unroll
-    for (int b = 1; b < 8; ++b) acc = cfma(mat(r * 8 + b), x[b], acc);
-    v[((r & 1) << P0) | (((r >> 1) & 1) << P1) | (((r >> 2) & 1) << P2)] = acc;
-  }
+  for (int b = 0; b < CUBE; ++b)
+    if (!((b >> J) & 1)) {
+      V<R>&a0 = v[b], &a1 = v[b | (1 << J)];
+      const R px = mul_rn(m10, a0.x), py = mul_rn(m10, a0.y);
+      a0.x = mul_rn(m00, a0.x);
+      a0.y = mul_rn(m00, a0.y);
+      a0.x = fma_rn(m01, a1.x, a0.x);
+      a0.y = fma_rn(m01, a1.y, a0.y);
+      a1.x = fma_rn(m11, a1.x, px);
+      a1.y = fma_rn(m11, a1.y, py);
+    }
 }
-
+template <class R, int J>
+__device__ __forceinline__ void chain_dense1_realcol(V<R> (&v)[CUBE], const V<R>* m) {
+  const R m00 = m[0].x, m01 = m[1].x, m11 = m[3].x;
+#pragma unroll
+  for (int b = 0; b < CUBE; ++b)
+    if (!((b >> J) & 1)) {
+      V<R>&a0 = v[b], &a1 = v[b | (1 << J)];
+      const R px = mul_rn(m00, a0.x), py = mul_rn(m00, a0.y);
+      a0.x = fma_rn(m01, a1.x, px);
+      a0.y = fma_rn(m01, a1.y, py);
+      a1.x = fma_rn(m11, a1.x, px);
+      a1.y = fma_rn(m11, a1.y, py);
+    }
+}
+template <class R, int J>
+__device__ __forceinline__ void chain_dense1_cross(V<R> (&v)[CUBE], const V<R>* m) {
+  const R m00 = m[0].x, i01 = m[1].y, i10 = m[2].y, m11 = m[3].x;
+#pragma unroll
+  for (int b = 0; b < CUBE; ++b)
+    if (!((b >> J) & 1)) {
+      V<R>&a0 = v[b], &a1 = v[b | (1 << J)];
+      const R px = -mul_rn(i10, a0.y), py = mul_rn(i10, a0.x);
+      a0.x = mul_rn(m00, a0.x);
+      a0.y = mul_rn(m00, a0.y);
+      a0.x = fma_rn(-i01, a1.y, a0.x);
+      a0.y = fma_rn(i01, a1.x, a0.y);
+      a1.x = fma_rn(m11, a1.x, px);
+      a1.y = fma_rn(m11, a1.y, py);
+    }
+}
+template <class R>
+__device__ __forceinline__ void phase_in_place(V<R>& u, V<R> c) {  // u = cmul(c, u)
+  const R t = mul_rn(c.y, u.y), s = mul_rn(c.y, u.x);
+  u.x = fma_rn(c.x, u.x, -t);
+  u.y = fma_rn(c.x, u.y, s);
+}
+template <class R, int J>
+__device__ __forceinline__ void chain_phase(V<R> (&v)[CUBE], V<R> c) {
+#pragma unroll
+  for (int b = 0; b < CUBE; ++b)
+    if (J < 0 || ((b >> (J < 0 ? 0 : J)) & 1)) phase_in_place<R>(v[b], c);
+}
+// u times (0, +1) (sx = sign bit, sy = 0) or (0, -1) (sx = 0, sy = sign bit)
+template <class V2>
+__device__ __forceinline__ void turn_in_place(V2& u, uint32_t sx, uint32_t sy) {
+  const auto x = u.x;
+  u.x = flip(u.y, sx);
+  u.y = flip(x, sy);
+}
+template <class R, int J>
+__device__ __forceinline__ void chain_turn(V<R> (&v)[CUBE], uint32_t sx, uint32_t sy) {
+#pragma unroll
+  for (int b = 0; b < CUBE; ++b)
+    if (J < 0 || ((b >> (J < 0 ? 0 : J)) & 1)) turn_in_place(v[b], sx, sy);
+}
+template <class R, int J>
+__device__ __forceinline__ void chain_rz(V<R> (&v)[CUBE], const V<R>* c) {
+  const V<R> c0 = c[0], c1 = c[1];
+#pragma unroll
+  for (int b = 0; b < CUBE; ++b) phase_in_place<R>(v[b], ((b >> J) & 1) ? c1 : c0);
+}
 template <class R, int X>
-__device__ __forceinline__ void chain_pairswap(V<R> (&v)[8], uint32_t em, uint32_t flags, V<R> ci, V<R> cj) {
+__device__ __forceinline__ void chain_swap(V<R> (&v)[CUBE], uint32_t em) {  // em: the smaller element of each pair
+#pragma unroll
+  for (int b = 0; b < CUBE; ++b)
+    if (b < (b ^ X))
+      if ((em >> b) & 1) {
+        const V<R> u = v[b];
+        v[b] = v[b ^ X];
+        v[b ^ X] = u;
+      }
+}
+template <class R, int X>
+__device__ __forceinline__ void chain_swapc(V<R> (&v)[CUBE], uint32_t em, uint32_t flags, const V<R>* c) {
+  const V<R> ci = c[0], cj = c[1];
   const bool ui = flags & 1, uj = (flags >> 1) & 1;
 #pragma unroll
-  for (int b = 0; b < 8; ++b)
+  for (int b = 0; b < CUBE; ++b)
     if ((em >> b) & 1) {
       const V<R> vi = v[b], vj = v[b ^ X];
       v[b] = ui ? vj : cmul(ci, vj);
       v[b ^ X] = uj ? vi : cmul(cj, vi);
     }
 }
+// the pending signs applied
+template <class R>
+__device__ __forceinline__ void chain_flush(V<R> (&v)[CUBE], uint32_t& pend) {
+  if (!pend) return;
+#pragma unroll
+  for (int b = 0; b < CUBE; ++b) {
+    const uint32_t s = (pend << (31 - b)) & 0x80000000u;
+    v[b].x = flip(v[b].x, s);
+    v[b].y = flip(v[b].y, s);
+  }
+  pend = 0;
+}
 
 template <class R>
-__device__ __forceinline__ V<R> phasepoly_elem(V<R> v, uint64_t i, const TileOp& op, const V<R>* cp, const uint32_t* up,
-                                               const uint64_t* pp, bool& changed) {
-  changed = false;
+__device__ __forceinline__ V<R> phasepoly_elem(V<R> v, uint64_t i, const OpArgs<R>& op, const PassParams<R>& P) {
   if (is_zero(v)) return v;
-  const uint32_t* u = up + op.up;
+  const uint32_t* u = P.upool + op.a[1];
+  const V<R>* cp = P.cpool + op.a[2];
+  const uint64_t* pp = P.ppool + op.a[3];
   const uint32_t bits = u[0];
   const bool use_table = u[1], s_one = u[2];
   const uint64_t constant = uint64_t(u[3]) | (uint64_t(u[4]) << 32);
-  const int nt = int(op.k);
+  const int nt = int(op.a[0]);
   const uint32_t* start = u + 5;
   const uint32_t* coeff = start + nt + 1;
   uint64_t f = constant;
   for (int tt = 0; tt < nt; ++tt) {
     int all = 1;
-    for (uint32_t l = start[tt]; l < start[tt + 1]; ++l) all &= __popcll(pp[op.gz + l] & i) & 1;
+    for (uint32_t l = start[tt]; l < start[tt + 1]; ++l) all &= __popcll(pp[l] & i) & 1;
     if (all) f += coeff[tt];
   }
   f &= (uint64_t(1) << bits) - 1;
   V<R> c;
   if (use_table) {
-    c = cp[op.cp + 1 + f];
+    c = cp[1 + f];
     if (is_one_v(c)) return v;
   } else {
     if (f == 0 && s_one) return v;
     const double2 rr = pass_root(f, bits);
     c.x = R(rr.x);
     c.y = R(rr.y);
-    if (!s_one) c = cmul(cp[op.cp], c);
+    if (!s_one) c = cmul(cp[0], c);
   }
-  changed = true;
   return cmul(c, v);
 }
 
 template <class R>
-__device__ void tile_chain(SwTile<R> t, uint32_t tsz, const TileOp* ops, const PassParams<R>& P, uint64_t base) {
-  const TileOp& head = ops[0];
-  const uint32_t nsub = head.k;
-  const uint8_t cpos[3] = {uint8_t(head.l0 & 0xff), uint8_t((head.l0 >> 8) & 0xff), uint8_t((head.l0 >> 16) & 0xff)};
-  uint32_t loff[8];
+__device__ __forceinline__ V<R> table_elem(V<R> v, uint32_t e, uint32_t xout, const OpArgs<R>& op, const PassParams<R>& P) {
+  const int k = int(op.a[0]);
+  if ((e & op.a[1]) != op.a[2]) return v;
+  const uint32_t* qp = P.upool + op.a[3];
+  const uint8_t* unit = reinterpret_cast<const uint8_t*>(qp + k);
+  uint32_t x = xout;
+  for (int j = 0; j < k; ++j)
+    if (qp[j] < 256) x |= ((e >> qp[j]) & 1u) << j;
+  return unit[x] ? v : cmul(P.cpool[op.a[4] + x], v);
+}
+
+// The chain whose head is op o.  gbase: the tile bits of the thread's cube (its index
+// spread over the tile bits outside the cube).
+template <class R>
+__device__ __forceinline__ void tile_chain(uint32_t tile, uint32_t o, uint32_t gbase, const OpArgs<R>* args,
+                                           const PassParams<R>& P, uint64_t base) {
+  V<R>* const t = shared_tile<R>() + tile;  // an index into the shared array, so that accesses stay in the shared space
+  const uint32_t nsub = P.head[o].em;
+  const uint32_t cbits = P.head[o].gml;  // cube bit j: byte j
+  const uint32_t gb = gbase;
+  uint32_t lb[CUBE_BITS], sb[CUBE_BITS];
 #pragma unroll
-  for (int b = 0; b < 8; ++b) loff[b] = ((b & 1u) << cpos[0]) | (((b >> 1) & 1u) << cpos[1]) | (((b >> 2) & 1u) << cpos[2]);
-  for (uint32_t grp = threadIdx.x; grp < (tsz >> 3); grp += blockDim.x) {
-    const uint32_t gb = insert_zeros32(grp, cpos, 3);
-    uint32_t e[8];
-    V<R> v[8];
+  for (int j = 0; j < CUBE_BITS; ++j) {
+    lb[j] = 1u << ((cbits >> (8 * j)) & 0xffu);
+    sb[j] = swz<R>(lb[j]);
+  }
+  const uint32_t sg = swz<R>(gb);
+  V<R> v[CUBE];
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      e[b] = gb | loff[b];
-      v[b] = t[e[b]];
-    }
-    for (uint32_t s = 0; s < nsub; ++s) {
-      const TileOp& op = ops[1 + s];
-      if ((base & op.gfix) != op.gval) continue;
-      // the op's constants (at most 64 of them: a 3-qubit matrix)
-      V<R> m[4];
-      switch (op.kind) {
-        case TK_DENSE1:
+  for (int b = 0; b < CUBE; ++b) {
+    uint32_t a = 0;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) m[i] = pconst(P, op.cp + i);
-          if (op.reg == 0) chain_dense1<R, 0>(v, m);
-          else if (op.reg == 1) chain_dense1<R, 1>(v, m);
-          else chain_dense1<R, 2>(v, m);
-          break;
-        case TK_DENSE2:
-          switch (op.reg) {  // ja | jb << 4
-            case 0x10: chain_dense2<R, 0, 1>(v, P, op.cp); break;
-            case 0x20: chain_dense2<R, 0, 2>(v, P, op.cp); break;
-            case 0x01: chain_dense2<R, 1, 0>(v, P, op.cp); break;
-            case 0x21: chain_dense2<R, 1, 2>(v, P, op.cp); break;
-            case 0x02: chain_dense2<R, 2, 0>(v, P, op.cp); break;
-            default: chain_dense2<R, 2, 1>(v, P, op.cp); break;
-          }
-          break;
-        case TK_FIBER:
-          switch (op.reg) {  // p0 | p1 << 4 | p2 << 8
-            case 0x210: chain_fiber<R, 0, 1, 2>(v, P, op.cp); break;
-            case 0x120: chain_fiber<R, 0, 2, 1>(v, P, op.cp); break;
-            case 0x201: chain_fiber<R, 1, 0, 2>(v, P, op.cp); break;
-            case 0x021: chain_fiber<R, 1, 2, 0>(v, P, op.cp); break;
-            case 0x102: chain_fiber<R, 2, 0, 1>(v, P, op.cp); break;
-            default: chain_fiber<R, 2, 1, 0>(v, P, op.cp); break;
-          }
-          break;
-        case TK_PAIRSWAP: {
-          if ((gb & op.gml) != op.gvl) break;
-          const V<R> ci = pconst(P, op.cp), cj = pconst(P, op.cp + 1);
-          const uint32_t em = op.reg >> 8;
-          switch (op.reg & 7) {
-            case 1: chain_pairswap<R, 1>(v, em, op.flags, ci, cj); break;
-            case 2: chain_pairswap<R, 2>(v, em, op.flags, ci, cj); break;
-            case 3: chain_pairswap<R, 3>(v, em, op.flags, ci, cj); break;
-            case 4: chain_pairswap<R, 4>(v, em, op.flags, ci, cj); break;
-            case 5: chain_pairswap<R, 5>(v, em, op.flags, ci, cj); break;
-            case 6: chain_pairswap<R, 6>(v, em, op.flags, ci, cj); break;
-            default: chain_pairswap<R, 7>(v, em, op.flags, ci, cj); break;
-          }
-          break;
+    for (int j = 0; j < CUBE_BITS; ++j)
+      if ((b >> j) & 1) a ^= sb[j];
+    v[b] = t[sg ^ a];
+  }
+  uint32_t pend = 0;  // elements whose sign is still to be flipped
+  OpHead hn = P.head[o + 1];
+  for (uint32_t s = o + 1; s <= o + nsub; ++s) {
+    const OpHead h = hn;
+    hn = P.head[min(s + 1, uint32_t(MAX_PASS_OPS - 1))];  // in flight while this op runs
+    const OpArgs<R>& op = args[s];
+    if ((h.kind & DK_COND) && (base & P.cond[s].gfix) != P.cond[s].gval) continue;  // uniform over the CTA
+    const bool on = (gb & h.gml) == h.gvl;
+    const uint32_t em = h.em;
+#define NCSIM_D1(j) \
+  case DK_D1 + j: chain_dense1<R, j>(v, op.c); break; \
+  case DK_D1R + j: chain_dense1_real<R, j>(v, op.c); break; \
+  case DK_D1RE + j: chain_dense1_realcol<R, j>(v, op.c); break; \
+  case DK_D1X + j: chain_dense1_cross<R, j>(v, op.c); break; \
+  case DK_D1E + j: chain_dense1_col<R, j, 2>(v, op.c); break; \
+  case DK_D1S + j: chain_dense1_col<R, j, 0>(v, op.c); break; \
+  case DK_D1SD + j: chain_dense1_col<R, j, 1>(v, op.c); break; \
+  case DK_PH + j: if (on) chain_phase<R, j>(v, op.c[0]); break; \
+  case DK_TURN + j: if (on) chain_turn<R, j>(v, op.a[0], op.a[1]); break; \
+  case DK_RZ + j: chain_rz<R, j>(v, op.c); break;
+#define NCSIM_SW(i, X) \
+  case DK_SWAP + i: if (on) chain_swap<R, X>(v, em); break; \
+  case DK_SWAPC + i: if (on) chain_swapc<R, X>(v, em & 0xffffu, em >> 16, op.c); break;
+    switch (h.kind & ~uint32_t(DK_COND)) {
+      NCSIM_D1(0)
+      NCSIM_D1(1)
+      NCSIM_D1(2)
+      NCSIM_D1(3)
+      NCSIM_SW(0, 1)
+      NCSIM_SW(1, 2)
+      NCSIM_SW(2, 4)
+      NCSIM_SW(3, 8)
+      NCSIM_SW(4, 3)
+      NCSIM_SW(5, 5)
+      NCSIM_SW(6, 9)
+      NCSIM_SW(7, 6)
+      NCSIM_SW(8, 10)
+      NCSIM_SW(9, 12)
+      case DK_PH_ALL:
+        if (on) chain_phase<R, -1>(v, op.c[0]);
+        break;
+      case DK_PH_MASK:
+        if (on) {
+          const V<R> c = op.c[0];
+#pragma unroll
+          for (int b = 0; b < CUBE; ++b)
+            if ((em >> b) & 1) phase_in_place<R>(v[b], c);
         }
-        case TK_DIAG_CONST: {
-          if ((gb & op.gml) != op.gvl) break;
-          const V<R> c = pconst(P, op.cp);
-          const uint32_t em = op.reg;  // the cube elements with the fixed pattern
+        break;
+      case DK_TURN_ALL:
+        if (on) chain_turn<R, -1>(v, op.a[0], op.a[1]);
+        break;
+      case DK_TURN_MASK:
+        if (on) {
+          const uint32_t sx = op.a[0], sy = op.a[1];
 #pragma unroll
-          for (int b = 0; b < 8; ++b)
-            if (((em >> b) & 1) && !is_zero(v[b])) v[b] = cmul(c, v[b]);
-          break;
+          for (int b = 0; b < CUBE; ++b)
+            if ((em >> b) & 1) turn_in_place(v[b], sx, sy);
         }
-        case TK_DIAG_1Q: {
-          const V<R> c0 = pconst(P, op.cp), c1 = pconst(P, op.cp + 1);
-          // the cube elements whose qubit bit is 1: from the cube, the group or the tile base
-          const uint32_t ones = (op.flags & 4) ? op.reg
-                              : (op.flags & 1) ? (((base >> op.l1) & 1) ? 0xffu : 0u)
-                                               : (((gb >> op.l0) & 1) ? 0xffu : 0u);
+        break;
+      case DK_SIGN:
+        if (on) pend ^= em;
+        break;
+      case DK_FLUSH: chain_flush<R>(v, pend); break;
+      case DK_RZ_OUT: chain_phase<R, -1>(v, op.c[on ? 1 : 0]); break;
+      case DK_TABLE: {
+        const int k = int(op.a[0]);
+        const uint32_t* qp = P.upool + op.a[3];
+        uint32_t xout = 0;
+        for (int j = 0; j < k; ++j)
+          if (qp[j] >= 256) xout |= uint32_t((base >> (qp[j] - 256)) & 1u) << j;
 #pragma unroll
-          for (int b = 0; b < 8; ++b)
-            if (!is_zero(v[b])) v[b] = cmul(((ones >> b) & 1) ? c1 : c0, v[b]);
-          break;
-        }
-        case TK_DIAG_TABLE: {
-          const int k = int(op.k);
-          const int nf = __popc(op.lfix);
-          const uint32_t* qp = P.upool + op.up;
-          const uint8_t* unit = reinterpret_cast<const uint8_t*>(qp + k + nf);
-          uint32_t xout = 0;
-          for (int j = 0; j < k; ++j)
-            if (qp[j] >= 256) xout |= uint32_t((base >> (qp[j] - 256)) & 1u) << j;
+        for (int b = 0; b < CUBE; ++b) {
+          uint32_t e = gb;
 #pragma unroll
-          for (int b = 0; b < 8; ++b) {
-            if ((e[b] & op.lfix) != op.lones) continue;
-            uint32_t x = xout;
-            for (int j = 0; j < k; ++j)
-              if (qp[j] < 256) x |= ((e[b] >> qp[j]) & 1u) << j;
-            if (unit[x]) continue;
-            if (!is_zero(v[b])) v[b] = cmul(pconst(P, op.cp + x), v[b]);
-          }
-          break;
+          for (int j = 0; j < CUBE_BITS; ++j)
+            if ((b >> j) & 1) e |= lb[j];
+          v[b] = table_elem<R>(v[b], e, xout, op, P);
         }
-        case TK_PHASEPOLY: {
-#pragma unroll
-          for (int b = 0; b < 8; ++b) {
-            bool ch;
-            v[b] = phasepoly_elem<R>(v[b], base | deposit(e[b], P.g), op, P.cpool, P.upool, P.ppool, ch);
-          }
-          break;
-        }
-        default: break;
+        break;
       }
-    }
+      case DK_POLY: {
 #pragma unroll
-    for (int b = 0; b < 8; ++b) t[e[b]] = v[b];
+        for (int b = 0; b < CUBE; ++b) {
+          uint32_t e = gb;
+#pragma unroll
+          for (int j = 0; j < CUBE_BITS; ++j)
+            if ((b >> j) & 1) e |= lb[j];
+          v[b] = phasepoly_elem<R>(v[b], base | deposit(e, P.g), op, P);
+        }
+        break;
+      }
+      default: break;
+    }
+#undef NCSIM_D1
+#undef NCSIM_SW
+  }
+  __syncwarp();  // registers of fewer than 2^9 amplitudes: two threads hold each cube and store the same values
+#pragma unroll
+  for (int b = 0; b < CUBE; ++b) {
+    uint32_t a = 0;
+#pragma unroll
+    for (int j = 0; j < CUBE_BITS; ++j)
+      if ((b >> j) & 1) a ^= sb[j];
+    t[sg ^ a] = v[b];
   }
 }
 
+// One thread per cube of a tile: 2^(T - CUBE_BITS) threads, at least a warp, at most 128; the
+// bound of three times that gives a thread 168 registers, what three CTAs per SM leave it.
+// (A bound of 128 threads and four CTAs, 128 registers, spills; the same 168 stated as
+// "three CTAs of 128" made ptxas copy the cube's registers at every op, 1.8 times the time.)
+constexpr int PASS_THREADS = 1 << (MAX_TILE_BITS - CUBE_BITS);
 template <class R>
-__global__ void __launch_bounds__(PASS_THREADS) k_plain_pass(const __grid_constant__ PassParams<R> P) {
-  extern __shared__ __align__(16) unsigned char pass_smem[];
+__global__ void __launch_bounds__(3 * PASS_THREADS) k_plain_pass(const __grid_constant__ PassParams<R> P) {
   const PassGeom& g = P.g;
   const uint32_t tsz = 1u << g.T;
-  V<R>* buf[2] = {reinterpret_cast<V<R>*>(pass_smem), reinterpret_cast<V<R>*>(pass_smem) + tsz};
-  __shared__ uint64_t dround[MAX_TILE_BITS > 9 ? (1 << MAX_TILE_BITS) / 32 : 32];
-  __shared__ TileOp s_ops[MAX_PASS_OPS];  // the ops, read from shared memory in the tile loop
-  const uint32_t nr = (tsz + blockDim.x - 1) / blockDim.x;  // element rounds per thread
-  for (uint32_t r = threadIdx.x; r < nr; r += blockDim.x) dround[r] = deposit(r * blockDim.x, g);
+  OpArgs<R>* const args = reinterpret_cast<OpArgs<R>*>(shared_tile<R>() + 2 * tsz);
+  uint16_t* const cubes = reinterpret_cast<uint16_t*>(args + P.nops);  // chain c, thread t: its cube at c * blockDim.x + t
+  __shared__ uint64_t dround[CUBE];
+  // element round r of a thread: elements threadIdx.x + r * blockDim.x
+  const uint32_t nr = (tsz + blockDim.x - 1) / blockDim.x;
+  if (threadIdx.x < nr) dround[threadIdx.x] = deposit(threadIdx.x * blockDim.x, g);
   {
-    const uint32_t words = P.nops * uint32_t(sizeof(TileOp) / 4);
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(P.ops);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(s_ops);
+    const uint32_t words = P.nops * uint32_t(sizeof(OpArgs<R>) / 16);
+    const uint4* src = reinterpret_cast<const uint4*>(P.args);
+    uint4* dst = reinterpret_cast<uint4*>(args);
     for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
   }
+  for (uint32_t o = 0; o < P.nops; ++o)
+    if (P.head[o].kind == DK_CHAIN) {
+      uint32_t gb = 0;
+      for (int i = 0; i < g.T - CUBE_BITS; ++i)
+        gb |= ((threadIdx.x >> i) & 1u) << ((P.args[o].a[i >> 2] >> (8 * (i & 3))) & 0xffu);
+      cubes[P.head[o].gvl * blockDim.x + threadIdx.x] = uint16_t(gb);
+    }
   const uint64_t dthread = deposit(threadIdx.x, g);
   __syncthreads();
-  auto load = [&](uint64_t tile, V<R>* dst) {
-    const V<R>* src = P.amp + (tile_base_of(tile, g) | dthread);
-    for (uint32_t r = 0; r < nr; ++r) {
-      const uint32_t e = threadIdx.x + r * blockDim.x;
-      if (e >= tsz) break;
-      const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(&SwTile<R>{dst}[e]));
-      if constexpr (sizeof(V<R>) == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + dround[r]) : "memory");
-      else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src + dround[r]) : "memory");
+  // f(element, its offset in the register) for the thread's elements of a tile
+  const auto elements = [&](auto f) {
+    if (nr == CUBE) {
+#pragma unroll
+      for (uint32_t r = 0; r < CUBE; ++r) f(threadIdx.x + r * blockDim.x, dround[r]);
+    } else {
+      for (uint32_t r = 0; r < nr; ++r) f(threadIdx.x + r * blockDim.x, dround[r]);
     }
+  };
+  const auto load = [&](uint64_t tile, uint32_t buf) {
+    const V<R>* src = P.amp + (tile_base_of(tile, g) | dthread);
+    V<R>* const dst = shared_tile<R>() + buf;
+    elements([&](uint32_t e, uint64_t off) {
+      const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst + swz<R>(e)));
+      if constexpr (sizeof(V<R>) == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + off) : "memory");
+      else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src + off) : "memory");
+    });
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   uint64_t tile = blockIdx.x;
-  if (tile < P.ntiles) load(tile, buf[0]);
-  for (uint32_t it = 0; tile < P.ntiles; ++it, tile += gridDim.x) {
-    const SwTile<R> t{buf[it & 1]};
+  if (tile < P.ntiles) load(tile, 0);
+  for (uint32_t buf = 0; tile < P.ntiles; buf ^= tsz, tile += gridDim.x) {
     const uint64_t next = tile + gridDim.x;
     if (next < P.ntiles) {
-      load(next, buf[(it & 1) ^ 1]);
+      load(next, buf ^ tsz);
       asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     } else {
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -611,33 +673,19 @@ __global__ void __launch_bounds__(PASS_THREADS) k_plain_pass(const __grid_consta
     __syncthreads();
     const uint64_t base = tile_base_of(tile, g);
     for (uint32_t o = 0; o < P.nops; ++o) {
-      const TileOp& op = s_ops[o];
-      if (op.kind == TK_CHAIN) {
-        tile_chain<R>(t, tsz, s_ops + o, P, base);
-        o += op.k;
-        __syncthreads();
-        continue;
-      }
-      if ((base & op.gfix) != op.gval) continue;  // uniform over the CTA
-      switch (op.kind) {
-        case TK_DENSE1: tile_dense1<R>(t, tsz, op, P.cpool); break;
-        case TK_DENSE2: tile_dense2<R>(t, tsz, op, P.cpool); break;
-        case TK_FIBER: tile_fiber<R, 3>(t, tsz, op, P.cpool, P.upool); break;
-        case TK_DIAG_CONST: tile_diag_const<R>(t, tsz, op, P.cpool, P.upool); break;
-        case TK_DIAG_1Q: tile_diag_1q<R>(t, tsz, op, P.cpool, base); break;
-        case TK_DIAG_TABLE: tile_diag_table<R>(t, tsz, op, P.cpool, P.upool, base); break;
-        case TK_PAIRSWAP: tile_pairswap<R>(t, tsz, op, P.cpool, P.upool); break;
-        case TK_PHASEPOLY: tile_phasepoly<R>(t, tsz, op, P.cpool, P.upool, P.ppool, base, dthread, dround); break;
-        default: break;
+      const OpHead& h = P.head[o];
+      if (h.kind == DK_CHAIN) {
+        tile_chain<R>(buf, o, cubes[h.gvl * blockDim.x + threadIdx.x], args, P, base);
+        o += h.em;
+      } else {  // DK_TILE_SWAP
+        if ((base & P.cond[o].gfix) != P.cond[o].gval) continue;
+        tile_pairswap<R>(SwTile<R>{shared_tile<R>() + buf}, tsz, args[o], P.cpool, P.upool);
       }
       __syncthreads();
     }
-    V<R>* dst = P.amp + (base | dthread);
-    for (uint32_t r = 0; r < nr; ++r) {
-      const uint32_t e = threadIdx.x + r * blockDim.x;
-      if (e >= tsz) break;
-      dst[dround[r]] = t[e];
-    }
+    V<R>* const dst = P.amp + (base | dthread);
+    const V<R>* const from = shared_tile<R>() + buf;
+    elements([&](uint32_t e, uint64_t off) { dst[off] = from[swz<R>(e)]; });
     __syncthreads();  // the buffer is refilled two tiles later
   }
 }
@@ -715,7 +763,7 @@ double touched_share(const GateForm& f, int precision) {
   }
 }
 
-GateForm form_of(const LoweredOp& op) {
+GateForm form_any(const LoweredOp& op) {
   GateForm f;
   f.qubits = op.qubits;
   switch (op.kind) {
@@ -735,10 +783,11 @@ GateForm form_of(const LoweredOp& op) {
         for (int x = 0; x < gd; ++x) d[x] = op.matrix[size_t(x) * gd + x];
         return form_diag_table(op.qubits, d);
       }
-      if (k > MAX_FIBER_K) return f;
+      // circuit text names dense matrices on one qubit only (every named gate on more is monomial)
+      if (k > 1) return f;
       f.tileable = true;
-      f.kind = k == 1 ? TK_DENSE1 : k == 2 ? TK_DENSE2 : TK_FIBER;
-      for (uint32_t q : op.qubits) f.moving |= uint64_t(1) << q;
+      f.kind = TK_DENSE1;
+      f.moving = uint64_t(1) << op.qubits[0];
       f.c = op.matrix;
       return f;
     }
@@ -809,12 +858,12 @@ GateForm form_of(const LoweredOp& op) {
   return f;
 }
 
-template <class R>
-V<R> cvt(const CplxD& c) {
-  V<R> r;
-  r.x = R(c.re);
-  r.y = R(c.im);
-  return r;
+// A gate with an infinite or NaN constant keeps its own kernel, which leaves zero amplitudes alone.
+GateForm form_of(const LoweredOp& op) {
+  GateForm f = form_any(op);
+  for (const auto& c : f.c)
+    if (!std::isfinite(c.re) || !std::isfinite(c.im)) f.tileable = false;
+  return f;
 }
 
 // the window's tile-local position of each global bit (-1: outside)
@@ -859,8 +908,7 @@ struct PlainPlan {
     bool pass = false;
     size_t gate = 0;              // direct: index into `gates`
     Window win;
-    std::vector<TileOp> ops;
-    uint32_t cbeg = 0, cend = 0;  // the pass's range of the constant pool
+    std::vector<DevOp> ops;
   };
   int precision = NCSIM_C128;
   std::vector<const LoweredOp*> gates;
@@ -906,28 +954,6 @@ TileOp encode(const GateForm& f, const Window& W, PlainPlan& P) {
       op.l0 = uint32_t(W.local[f.qubits[0]]);
       for (auto& c : f.c) push_c(c);
       break;
-    case TK_DENSE2:
-      op.l0 = uint32_t(W.local[f.qubits[0]]);
-      op.l1 = uint32_t(W.local[f.qubits[1]]);
-      for (auto& c : f.c) push_c(c);
-      break;
-    case TK_FIBER: {
-      const int k = int(f.qubits.size());
-      op.k = uint32_t(k);
-      std::vector<uint32_t> lp;
-      for (uint32_t q : f.qubits) lp.push_back(uint32_t(W.local[q]));
-      std::vector<uint32_t> sorted = lp;
-      std::sort(sorted.begin(), sorted.end());
-      for (uint32_t v : sorted) P.upool.push_back(v);
-      for (int b = 0; b < (1 << k); ++b) {
-        uint32_t o = 0;
-        for (int j = 0; j < k; ++j)
-          if ((b >> j) & 1) o |= 1u << lp[j];
-        P.upool.push_back(o);
-      }
-      for (auto& c : f.c) push_c(c);
-      break;
-    }
     case TK_DIAG_CONST:
     case TK_PAIRSWAP: {
       op.lfix = local_mask(W, f.fixmask);
@@ -936,8 +962,6 @@ TileOp encode(const GateForm& f, const Window& W, PlainPlan& P) {
       op.gval = f.ones & out;
       op.lx = local_mask(W, f.xmask);
       op.flags = f.flags;
-      for (int b = 0; b < MAX_TILE_BITS; ++b)
-        if ((op.lfix >> b) & 1) P.upool.push_back(uint32_t(b));
       for (auto& c : f.c) push_c(c);
       break;
     }
@@ -960,8 +984,6 @@ TileOp encode(const GateForm& f, const Window& W, PlainPlan& P) {
       op.gfix = f.fixmask & out;
       op.gval = f.fixmask & out;
       for (uint32_t q : f.qubits) P.upool.push_back(W.local[q] >= 0 ? uint32_t(W.local[q]) : 256u + q);
-      for (int b = 0; b < MAX_TILE_BITS; ++b)
-        if ((op.lfix >> b) & 1) P.upool.push_back(uint32_t(b));
       const size_t nb = f.unit.size();
       std::vector<uint32_t> words((nb + 3) / 4, 0);
       for (size_t x = 0; x < nb; ++x) words[x / 4] |= uint32_t(f.unit[x]) << (8 * (x % 4));
@@ -991,98 +1013,229 @@ TileOp encode(const GateForm& f, const Window& W, PlainPlan& P) {
 }
 
 // tile bits an op couples (0 for the ops that act on each element alone)
-uint32_t coupled_bits(const TileOp& op, const std::vector<uint32_t>& upool) {
+uint32_t coupled_bits(const TileOp& op) {
   switch (op.kind) {
     case TK_DENSE1: return 1u << op.l0;
-    case TK_DENSE2: return (1u << op.l0) | (1u << op.l1);
-    case TK_FIBER: return (1u << upool[op.up]) | (1u << upool[op.up + 1]) | (1u << upool[op.up + 2]);
     case TK_PAIRSWAP: return op.lx;
     default: return 0;
   }
 }
 
-// Groups a pass's ops into chains: maximal runs of two or more consecutive ops
-// whose coupled bits fit in one cube of three tile bits.
-std::vector<TileOp> chainify(const std::vector<TileOp>& ops, const std::vector<uint32_t>& upool, int T) {
-  std::vector<TileOp> out;
+// the exchange of a chain spans one or two cube bits; wider ones sweep the tile by themselves
+bool chainable(const TileOp& op) { return op.kind != TK_PAIRSWAP || __builtin_popcount(op.lx) <= 2; }
+
+// Orders a chain's thread bits: the lowest SB (a quarter warp of 16-byte elements, half a
+// warp of 8-byte ones) on tile bits of distinct residues mod SB, so that their accesses
+// fall into distinct banks (swz), the rest ascending.
+void thread_bits(int T, uint32_t cmask, int SB, uint8_t* at) {
+  std::vector<int> free_bits;
+  for (int b = 0; b < T; ++b)
+    if (!((cmask >> b) & 1)) free_bits.push_back(b);
+  std::vector<int> first, rest;
+  uint32_t seen = 0;
+  for (int b : free_bits) {
+    const uint32_t r = 1u << (b % SB);
+    if (int(first.size()) < SB && !(seen & r)) first.push_back(b), seen |= r;
+    else rest.push_back(b);
+  }
+  int i = 0;
+  for (int b : first) at[i++] = uint8_t(b);
+  for (int b : rest) at[i++] = uint8_t(b);
+}
+
+// Groups a pass's ops into chains: maximal runs of consecutive ops whose coupled bits fit in
+// one cube of CUBE_BITS tile bits, each op encoded against its cube.
+std::vector<DevOp> chainify(const std::vector<TileOp>& ops, int T, PlainPlan& P) {
+  std::vector<DevOp> out;
+  const auto cst = [&](uint32_t i) { return make_double2(P.cpool[2 * size_t(i)], P.cpool[2 * size_t(i) + 1]); };
+  uint32_t chains = 0;
   size_t i = 0;
   while (i < ops.size()) {
+    if (!chainable(ops[i])) {
+      const TileOp& op = ops[i++];
+      DevOp d{};
+      d.h.kind = DK_TILE_SWAP;
+      d.g.gfix = op.gfix;
+      d.g.gval = op.gval;
+      d.x.a[0] = uint32_t(__builtin_popcount(op.lfix));
+      d.x.a[1] = uint32_t(P.upool.size());
+      for (int b = 0; b < T; ++b)
+        if ((op.lfix >> b) & 1) P.upool.push_back(uint32_t(b));
+      d.x.a[2] = op.flags;
+      d.x.a[3] = op.lx;
+      d.x.a[4] = op.lones;
+      d.x.a[5] = op.cp;
+      out.push_back(d);
+      continue;
+    }
     uint32_t C = 0;
     size_t j = i;
-    while (j < ops.size()) {
-      const uint32_t need = coupled_bits(ops[j], upool);
-      if (__builtin_popcount(C | need) > 3) break;
+    while (j < ops.size() && chainable(ops[j])) {
+      const uint32_t need = coupled_bits(ops[j]);
+      if (__builtin_popcount(C | need) > CUBE_BITS) break;
       C |= need;
       ++j;
     }
-    if (j - i < 2 || T < 3) {
-      out.push_back(ops[i]);
-      i = i + 1;
-      continue;
-    }
-    for (int b = 0; b < T && __builtin_popcount(C) < 3; ++b) C |= 1u << b;
-    int cpos[3], nc = 0;
+    // filled with the highest free bits: the low ones stay with the lanes
+    for (int b = T - 1; b >= 0 && __builtin_popcount(C) < CUBE_BITS; --b) C |= 1u << b;
+    int cpos[CUBE_BITS], nc = 0;
     for (int b = 0; b < T; ++b)
       if ((C >> b) & 1) cpos[nc++] = b;
     auto cube = [&](uint32_t l) {
-      for (int q = 0; q < 3; ++q)
-        if (cpos[q] == int(l)) return uint32_t(q);
+      for (uint32_t q = 0; q < CUBE_BITS; ++q)
+        if (cpos[q] == int(l)) return q;
       return 0u;
     };
-    const uint32_t cmask = (1u << cpos[0]) | (1u << cpos[1]) | (1u << cpos[2]);
-    uint32_t loff[8];
-    for (int b = 0; b < 8; ++b)
-      loff[b] = ((b & 1u) << cpos[0]) | (((b >> 1) & 1u) << cpos[1]) | (((b >> 2) & 1u) << cpos[2]);
+    uint32_t loff[CUBE] = {};
+    for (int b = 0; b < CUBE; ++b)
+      for (int q = 0; q < CUBE_BITS; ++q)
+        if ((b >> q) & 1) loff[b] |= 1u << cpos[q];
     // the cube elements b whose cube bits match the op's fixed pattern there
     auto elements = [&](uint32_t lfix, uint32_t lones) {
       uint32_t em = 0;
-      for (int b = 0; b < 8; ++b)
-        if ((loff[b] & lfix) == (lones & cmask)) em |= 1u << b;
+      for (int b = 0; b < CUBE; ++b)
+        if ((loff[b] & lfix) == (lones & C & lfix)) em |= 1u << b;
       return em;
     };
-    TileOp head{};
-    head.kind = TK_CHAIN;
-    head.k = uint32_t(j - i);
-    head.l0 = uint32_t(cpos[0]) | (uint32_t(cpos[1]) << 8) | (uint32_t(cpos[2]) << 16);
+    DevOp head{};
+    head.h.kind = DK_CHAIN;
+    for (int q = 0; q < CUBE_BITS; ++q) head.h.gml |= uint32_t(cpos[q]) << (8 * q);
+    uint8_t tb[MAX_TILE_BITS] = {};
+    thread_bits(T, C, P.precision == NCSIM_C128 ? 3 : 4, tb);
+    for (int q = 0; q < T - CUBE_BITS; ++q) head.x.a[q >> 2] |= uint32_t(tb[q]) << (8 * (q & 3));
+    head.h.gvl = chains++;
+    const size_t at_head = out.size();
     out.push_back(head);
+    bool pending = false;
+    const auto flush = [&] {
+      if (!pending) return;
+      DevOp d{};
+      d.h.kind = DK_FLUSH;
+      out.push_back(d);
+      pending = false;
+    };
     for (size_t o = i; o < j; ++o) {
-      TileOp op = ops[o];
+      const TileOp& op = ops[o];
+      DevOp d{};
+      d.g.gfix = op.gfix;
+      d.g.gval = op.gval;
+      d.h.gml = op.lfix & ~C;
+      d.h.gvl = op.lones & ~C;
+      if (op.kind == TK_DENSE1 || op.kind == TK_PAIRSWAP) flush();
       switch (op.kind) {
-        case TK_DENSE1: op.reg = cube(op.l0); break;
-        case TK_DENSE2: op.reg = cube(op.l0) | (cube(op.l1) << 4); break;
-        case TK_FIBER: {
-          uint32_t r = 0;
-          for (int q = 0; q < 3; ++q) r |= cube(uint32_t(__builtin_ctz(upool[op.up + 3 + (1u << q)]))) << (4 * q);
-          op.reg = r;
+        case TK_DENSE1: {
+          for (int q = 0; q < 4; ++q) d.x.c[q] = cst(op.cp + uint32_t(q));
+          const double2 m00 = d.x.c[0], m01 = d.x.c[1], m10 = d.x.c[2], m11 = d.x.c[3];
+          const bool real = m00.y == 0.0 && m01.y == 0.0 && m10.y == 0.0 && m11.y == 0.0;
+          const bool col = m00.x == m10.x && m00.y == m10.y;
+          const bool half = m00.x == 0.5 && m10.x == 0.5;
+          DevKind kind = DK_D1;
+          if (real) kind = col ? DK_D1RE : DK_D1R;
+          else if (m00.y == 0.0 && m11.y == 0.0 && m01.x == 0.0 && m10.x == 0.0) kind = DK_D1X;
+          else if (col) kind = DK_D1E;
+          else if (half && m00.y == 0.5 && m10.y == -0.5) kind = DK_D1S;
+          else if (half && m00.y == -0.5 && m10.y == 0.5) kind = DK_D1SD;
+          d.h.kind = kind + cube(op.l0);
+          d.g.gfix = d.g.gval = 0;
+          d.h.gml = d.h.gvl = 0;
           break;
         }
-        case TK_PAIRSWAP: {
-          uint32_t r = 0;
-          for (int b = 0; b < T; ++b)
-            if ((op.lx >> b) & 1) r |= 1u << cube(uint32_t(b));
-          op.reg = r | (elements(op.lfix, op.lones) << 8);
-          op.gml = op.lfix & ~cmask;
-          op.gvl = op.lones & ~cmask;
-          break;
-        }
-        case TK_DIAG_CONST:
-          op.reg = elements(op.lfix, op.lones);
-          op.gml = op.lfix & ~cmask;
-          op.gvl = op.lones & ~cmask;
-          break;
-        case TK_DIAG_1Q:
-          if (!(op.flags & 1) && ((cmask >> op.l0) & 1)) {
-            op.flags |= 4;
-            op.reg = elements(1u << op.l0, 1u << op.l0);
+        case TK_DIAG_CONST: {
+          const double2 c = cst(op.cp);
+          d.h.em = elements(op.lfix, op.lones);
+          int half = -1;  // the cube bit whose upper half the mask is
+          for (int q = 0; q < CUBE_BITS; ++q)
+            if (d.h.em == elements(1u << cpos[q], 1u << cpos[q])) half = q;
+          const bool all = d.h.em == (1u << CUBE) - 1;
+          if (c.x == -1.0 && c.y == 0.0) {
+            d.h.kind = DK_SIGN;
+            pending = true;
+          } else if (c.x == 0.0 && (c.y == 1.0 || c.y == -1.0)) {
+            d.h.kind = half >= 0 ? DK_TURN + uint32_t(half) : all ? DK_TURN_ALL : DK_TURN_MASK;
+            d.x.a[0] = c.y > 0 ? 0x80000000u : 0u;  // i u = (-u.y, u.x)
+            d.x.a[1] = c.y > 0 ? 0u : 0x80000000u;  // -i u = (u.y, -u.x)
+          } else {
+            d.h.kind = half >= 0 ? DK_PH + uint32_t(half) : all ? DK_PH_ALL : DK_PH_MASK;
+            d.x.c[0] = c;
           }
           break;
-        default: break;
+        }
+        case TK_DIAG_1Q:
+          d.x.c[0] = cst(op.cp);
+          d.x.c[1] = cst(op.cp + 1);
+          d.h.gml = d.h.gvl = 0;
+          if (op.flags & 1) {  // outside the window: one of the two phases, by the bit of the tile's base
+            d.h.kind = DK_PH_ALL | DK_COND;
+            d.g.gfix = uint64_t(1) << op.l1;
+            d.g.gval = 0;
+            out.push_back(d);
+            d.x.c[0] = d.x.c[1];
+            d.g.gval = d.g.gfix;
+          } else if ((C >> op.l0) & 1) {
+            d.h.kind = DK_RZ + cube(op.l0);
+          } else {
+            d.h.kind = DK_RZ_OUT;
+            d.h.gml = d.h.gvl = 1u << op.l0;
+          }
+          break;
+        case TK_PAIRSWAP: {
+          uint32_t x = 0;
+          for (int b = 0; b < T; ++b)
+            if ((op.lx >> b) & 1) x |= 1u << cube(uint32_t(b));
+          uint32_t xi = 0;
+          while (SWAP_X[xi] != x) ++xi;
+          const uint32_t lead = elements(op.lfix, op.lones);
+          if ((op.flags & 3) == 3) {
+            d.h.kind = DK_SWAP + xi;
+            for (uint32_t b = 0; b < CUBE; ++b)
+              if ((lead >> b) & 1) d.h.em |= 1u << std::min(b, b ^ x);
+          } else {
+            d.h.kind = DK_SWAPC + xi;
+            d.h.em = lead | (op.flags << 16);
+            d.x.c[0] = cst(op.cp);
+            d.x.c[1] = cst(op.cp + 1);
+          }
+          break;
+        }
+        case TK_DIAG_TABLE:
+          d.h.kind = DK_TABLE;
+          d.h.gml = d.h.gvl = 0;  // the fixed bits are compared per element
+          d.x.a[0] = op.k;
+          d.x.a[1] = op.lfix;
+          d.x.a[2] = op.lones;
+          d.x.a[3] = op.up;
+          d.x.a[4] = op.cp;
+          break;
+        default:  // TK_PHASEPOLY
+          d.h.kind = DK_POLY;
+          d.h.gml = d.h.gvl = 0;
+          d.x.a[0] = op.k;
+          d.x.a[1] = op.up;
+          d.x.a[2] = op.cp;
+          d.x.a[3] = uint32_t(op.gz);
+          break;
       }
-      out.push_back(op);
+      if (d.g.gfix) d.h.kind |= DK_COND;
+      out.push_back(d);
     }
+    flush();
+    out[at_head].h.em = uint32_t(out.size() - at_head - 1);
     i = j;
   }
   return out;
+}
+
+// whether an op of this kind carries constants (else words)
+bool has_constants(uint32_t kind) {
+  kind &= ~uint32_t(DK_COND);
+  return (kind >= DK_D1 && kind <= DK_PH_MASK) || (kind >= DK_RZ && kind <= DK_RZ_OUT) || (kind >= DK_SWAPC && kind < DK_TABLE);
+}
+void put_args(OpArgs<double>& to, const DevOp& from) { to = from.x; }
+void put_args(OpArgs<float>& to, const DevOp& from) {
+  to = OpArgs<float>{};
+  for (int q = 0; q < 8; ++q) to.a[q] = from.x.a[q];
+  if (has_constants(from.h.kind))
+    for (int q = 0; q < 4; ++q) to.c[q] = make_float2(float(from.x.c[q].x), float(from.x.c[q].y));
 }
 
 }  // namespace
@@ -1098,7 +1251,8 @@ std::shared_ptr<PlainPlan> plan_plain_passes(uint32_t n, int precision, const st
   std::vector<GateForm> forms(gates.size());
   for (size_t i = 0; i < gates.size(); ++i) forms[i] = form_of(*gates[i]);
   std::vector<size_t> cur;
-  uint64_t moving = 0;
+  const uint64_t low = n > uint32_t(FREE_WINDOW_QUBITS) ? (uint64_t(1) << LOW_WINDOW_BITS) - 1 : 0;
+  uint64_t moving = low;  // the window's qubits so far
   auto flush = [&] {
     if (cur.empty()) return;
     // a pass reads and writes the whole register once; gates whose own kernels
@@ -1116,17 +1270,15 @@ std::shared_ptr<PlainPlan> plan_plain_passes(uint32_t n, int precision, const st
       it.pass = true;
       it.win = make_window(n, T, moving);
       std::vector<TileOp> ops;
-      it.cbeg = uint32_t(P->cpool.size() / 2);
       for (size_t i : cur) ops.push_back(encode(forms[i], it.win, *P));
-      it.cend = uint32_t(P->cpool.size() / 2);
-      it.ops = chainify(ops, P->upool, it.win.g.T);
+      it.ops = chainify(ops, it.win.g.T, *P);
       if (it.ops.size() > size_t(MAX_PASS_OPS)) throw Error(NCSIM_ERR_INVALID, "tiled pass: too many ops");
       P->passes += 1;
       P->pass_gates += cur.size();
       P->items.push_back(std::move(it));
     }
     cur.clear();
-    moving = 0;
+    moving = low;
   };
   for (size_t i = 0; i < gates.size(); ++i) {
     const GateForm& f = forms[i];
@@ -1138,8 +1290,9 @@ std::shared_ptr<PlainPlan> plan_plain_passes(uint32_t n, int precision, const st
       P->items.push_back(it);
       continue;
     }
-    // chains add at most one head per op: a pass of MAX_PASS_OPS / 2 gates fits in shared memory
-    if (__builtin_popcountll(moving | f.moving) > T || cur.size() >= size_t(MAX_PASS_OPS / 2)) flush();
+    // a gate makes at most three ops (a chain's head, two phases or a flush and the op; a chain's last
+    // flush comes with a sign, which is one op): a pass of MAX_PASS_OPS / 3 gates fits
+    if (__builtin_popcountll(moving | f.moving) > T || cur.size() >= size_t(MAX_PASS_OPS / 3)) flush();
     cur.push_back(i);
     moving |= f.moving;
   }
@@ -1148,40 +1301,30 @@ std::shared_ptr<PlainPlan> plan_plain_passes(uint32_t n, int precision, const st
   return P;
 }
 
-// passes, gates in passes, chains and ops in chains, and gates left to their own kernels
-std::string plain_plan_summary(const PlainPlan& P) {
-  size_t chains = 0, chained = 0, direct = 0;
-  for (const auto& it : P.items) {
-    if (!it.pass) {
-      ++direct;
-      continue;
-    }
-    for (const auto& op : it.ops)
-      if (op.kind == TK_CHAIN) ++chains, chained += op.k;
-  }
-  return "passes " + std::to_string(P.passes) + ", gates in passes " + std::to_string(P.pass_gates) + ", chains " +
-         std::to_string(chains) + " holding " + std::to_string(chained) + " ops, own kernels " + std::to_string(direct);
-}
-
-size_t plain_plan_passes(const PlainPlan& P) { return P.passes; }
-size_t plain_plan_pass_gates(const PlainPlan& P) { return P.pass_gates; }
-
 void apply_lowered(ncsim_state* s, const LoweredOp& op);
 
 template <class R>
 void launch_pass(ncsim_state* s, const PlainPlan& P, const PlainPlan::Item& it) {
-  PassParams<R> pp{};
+  PassParams<R> pp;
   pp.amp = reinterpret_cast<V<R>*>(s->amp);
   pp.g = it.win.g;
   pp.ntiles = s->len >> it.win.g.T;
   pp.nops = uint32_t(it.ops.size());
-  std::copy(it.ops.begin(), it.ops.end(), pp.ops);
-
+  pp.nchains = 0;
+  for (size_t i = 0; i < it.ops.size(); ++i) {
+    pp.head[i] = it.ops[i].h;
+    pp.cond[i] = it.ops[i].g;
+    put_args(pp.args[i], it.ops[i]);
+    pp.nchains += it.ops[i].h.kind == DK_CHAIN;
+  }
   pp.upool = P.d_upool;
   pp.ppool = P.d_ppool;
   // the complex pool as this precision's values
   pp.cpool = reinterpret_cast<const V<R>*>(P.d_cpool);
-  const size_t smem = 2 * (size_t(1) << it.win.g.T) * sizeof(V<R>);
+  const int T = it.win.g.T;
+  const unsigned threads = std::max(32u, 1u << (T - CUBE_BITS));
+  const size_t smem = 2 * (size_t(1) << T) * sizeof(V<R>) + it.ops.size() * sizeof(OpArgs<R>) +
+                      size_t(pp.nchains) * threads * sizeof(uint16_t);
   {
     // the kernel's shared-memory limit, set once per device and precision (host threads may race here)
     static std::mutex mu;
@@ -1189,14 +1332,18 @@ void launch_pass(ncsim_state* s, const PlainPlan& P, const PlainPlan::Item& it) 
     std::lock_guard<std::mutex> lk(mu);
     const int dev = s->device;
     if (dev < 0 || dev >= 64 || !done[dev][sizeof(R) == 8]) {
-      NCSIM_CUDA(cudaFuncSetAttribute(k_plain_pass<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(2 * (size_t(1) << MAX_TILE_BITS) * sizeof(V<R>))));
+      NCSIM_CUDA(cudaFuncSetAttribute(
+          k_plain_pass<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+          int(2 * (size_t(1) << MAX_TILE_BITS) * sizeof(V<R>) + MAX_PASS_OPS * sizeof(OpArgs<R>) +
+              MAX_PASS_CHAINS * (1 << (MAX_TILE_BITS - CUBE_BITS)) * sizeof(uint16_t))));
       if (dev >= 0 && dev < 64) done[dev][sizeof(R) == 8] = true;
     }
   }
-  const uint64_t grid = std::min<uint64_t>(pp.ntiles, uint64_t(sm_count()) * (sizeof(R) == 8 ? 1 : 2));
+  int per_sm = 1;
+  NCSIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_plain_pass<R>, int(threads), smem));
+  const uint64_t grid = std::min<uint64_t>(pp.ntiles, uint64_t(sm_count()) * uint64_t(std::max(per_sm, 1)));
   ProfScope ps(s, K_PLAIN_PASS, 2.0 * double(s->len) * double(s->elem_bytes()));
-  k_plain_pass<R><<<unsigned(grid), PASS_THREADS, smem, s->stream>>>(pp);
+  k_plain_pass<R><<<unsigned(grid), threads, smem, s->stream>>>(pp);
   NCSIM_LAUNCHED("k_plain_pass");
 }
 
