@@ -26,6 +26,7 @@ SOURCES = [
     "csrc/batch_plan.cpp",
     "csrc/sparse.cu",
     "csrc/sparse_wide.cu",
+    "csrc/sparse_run.cu",
     "csrc/frames.cu",
     "csrc/frames_plan.cpp",
     "csrc/host/ir.cpp",
@@ -37,6 +38,7 @@ WORKLOAD_SOURCES = ["csrc/workloads/workloads.cpp"]
 HEADERS = [
     "csrc/engine.cuh",
     "csrc/sparse_common.cuh",
+    "csrc/sparse_run.hpp",
     "csrc/host_math.hpp",
     "csrc/fused_plan.hpp",
     "csrc/batch_plan.hpp",

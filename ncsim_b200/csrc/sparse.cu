@@ -13,6 +13,7 @@
 // added on the host in a fixed order; Born sampling takes the cumulative
 // weights in entry order on the host, as sparse.rs:407-424 does.
 #include "sparse_common.cuh"
+#include "sparse_run.hpp"
 
 using namespace ncsim;
 
@@ -139,98 +140,6 @@ __global__ void k_sp_tensor(const uint64_t* ka, const double2* va, uint64_t ma, 
     const uint64_t jb = i / ma, ia = i - jb * ma;
     okey[i] = ka[ia] | (na >= 64 ? 0 : (kb[jb] << na));
     oamp[i] = zmul(va[ia], vb[jb]);
-  }
-}
-
-// ---- a run of one-to-one ops in one pass ----
-// Monomial gates, diagonals and Paulis map each entry to one entry, so a run of
-// them is applied entry by entry: one thread walks the run's op list with its
-// entry in registers (one launch and one read and write of the entries per run).
-enum : uint32_t { RUN_MONO = 0, RUN_POLY = 1, RUN_PAULI = 2 };
-struct RunOp {
-  uint32_t type;
-  uint32_t k;        // MONO: qubits; POLY: terms
-  uint8_t q[SP_MAX_K];
-  uint16_t pad;
-  uint32_t off;      // MONO: first pattern in image/phase/unit; POLY: first term in start
-  uint32_t bits;     // POLY
-  uint32_t flags;    // POLY: bit 0 scalar is one, bit 1 phasor table; PAULI: the phase
-  uint32_t toff;     // POLY: first entry of its phasor table in RunData::table
-  uint64_t x, z;     // PAULI; POLY: x = constant
-  double2 scalar;    // POLY
-  // MONO on at most 3 qubits: the 8 images (16 bits each: patterns 0..3, 4..7) and unit flags
-  // (byte x: the phase of pattern x is exactly 1), packed on the host
-  uint64_t img_lo, img_hi, unit8;
-};
-struct RunData {
-  const RunOp* ops;
-  uint32_t nops;
-  const uint16_t* image;  // monomial tables (image, phase, unit share the op's offset)
-  const double2* phase;
-  const uint8_t* unit;
-  const double2* table;   // polynomial phasor tables
-  const uint32_t* start;  // polynomial term starts (absolute indices into par)
-  const uint64_t* par;
-  const uint64_t* coeff;
-  const uint64_t* and_mask;  // per term (aligned with coeff): the AND of single-bit parities, or 0
-};
-// The block stages the run's op descriptors RUN_STAGE at a time in shared
-// memory, so each thread's walk reads them as broadcasts instead of a chain of
-// dependent global loads per op; monomials on at most 3 qubits carry their image
-// and unit tables in the descriptor, a wider monomial's three table loads issue
-// together, and a phase polynomial's terms are loaded 32 at a time by the warp.
-// Every lane walks the ops (lanes past the last entry on a dummy entry) so that
-// the warp's shuffles see all 32 lanes.
-constexpr uint32_t RUN_STAGE = SP_THREADS;
-__global__ void __launch_bounds__(SP_THREADS) k_sp_run(uint64_t* key, double2* amp, uint64_t m, RunData d) {
-  __shared__ RunOp s_op[RUN_STAGE];
-  for (uint64_t base = uint64_t(blockIdx.x) * blockDim.x; base < m; base += uint64_t(gridDim.x) * blockDim.x) {
-    const uint64_t i = base + threadIdx.x;
-    const bool live = i < m;
-    uint64_t kk = live ? key[i] : 0;
-    double2 a = live ? amp[i] : make_double2(0.0, 0.0);
-    for (uint32_t o0 = 0; o0 < d.nops; o0 += RUN_STAGE) {
-      const uint32_t cnt = min(RUN_STAGE, d.nops - o0);
-      __syncthreads();
-      if (threadIdx.x < cnt) s_op[threadIdx.x] = d.ops[o0 + threadIdx.x];
-      __syncthreads();
-      for (uint32_t c = 0; c < cnt; ++c) {
-        const RunOp& op = s_op[c];
-        if (op.type == RUN_MONO) {
-          const uint32_t k = op.k;
-          uint32_t x = 0;
-          for (uint32_t j = 0; j < k; ++j) x |= uint32_t((kk >> op.q[j]) & 1u) << j;
-          uint32_t y;
-          bool unit;
-          double2 ph = make_double2(1.0, 0.0);
-          if (k <= 3) {
-            y = uint32_t((x < 4 ? op.img_lo : op.img_hi) >> (16 * (x & 3))) & 0xffffu;
-            unit = (op.unit8 >> (8 * x)) & 1u;
-            if (!unit) ph = d.phase[op.off + x];
-          } else {
-            y = d.image[op.off + x];
-            unit = d.unit[op.off + x];
-            ph = d.phase[op.off + x];
-          }
-          if (!unit) a = zmul(ph, a);
-          if (y != x)
-            for (uint32_t j = 0; j < k; ++j)
-              kk = (kk & ~(uint64_t(1) << op.q[j])) | (uint64_t((y >> j) & 1u) << op.q[j]);
-        } else if (op.type == RUN_POLY) {
-          const uint64_t f =
-              poly_sum_warp(kk, op.k, op.x, d.start + op.off, d.par, d.coeff + op.off, d.and_mask + op.off);
-          poly_finish(f, a, op.bits, op.flags & 1u, op.scalar, (op.flags >> 1) & 1u, d.table + op.toff);
-        } else {
-          const uint32_t ph = (op.flags + 2u * uint32_t(__popcll(op.z & kk))) & 3u;
-          if (ph) a = ipow(a, ph);
-          kk ^= op.x;
-        }
-      }
-    }
-    if (live) {
-      key[i] = kk;
-      amp[i] = a;
-    }
   }
 }
 
@@ -546,120 +455,6 @@ void sp_matrix(ncsim_sparse* s, const std::vector<uint32_t>& qubits, const std::
   dfree(off, st);
   sp_normalize_from(s, okey, oamp, total);
 }
-
-// the host side of a run: ops and their tables, launched in one kernel
-struct RunBuilder {
-  std::vector<RunOp> ops;
-  std::vector<uint16_t> image;
-  std::vector<double2> phase;
-  std::vector<uint8_t> unit;
-  std::vector<double2> table;
-  std::vector<uint32_t> start;
-  std::vector<uint64_t> par, coeff, and_mask;
-  bool moves = false;
-
-  bool empty() const { return ops.empty(); }
-  // empties the builder and keeps its buffers' capacity for the next run
-  void reset() {
-    ops.clear();
-    image.clear();
-    phase.clear();
-    unit.clear();
-    table.clear();
-    start.clear();
-    par.clear();
-    coeff.clear();
-    and_mask.clear();
-    moves = false;
-  }
-  void add_mono(const std::vector<uint32_t>& qubits, const std::vector<uint32_t>& img, const std::vector<CplxD>& ph) {
-    RunOp op{};
-    op.type = RUN_MONO;
-    op.k = uint32_t(qubits.size());
-    for (uint32_t j = 0; j < op.k; ++j) op.q[j] = uint8_t(qubits[j]);
-    op.off = uint32_t(image.size());
-    for (size_t x = 0; x < img.size(); ++x) {
-      image.push_back(uint16_t(img[x]));
-      phase.push_back(make_double2(ph[x].re, ph[x].im));
-      const bool one = ph[x].re == 1.0 && ph[x].im == 0.0;
-      unit.push_back(one);
-      moves |= img[x] != x;
-      if (op.k <= 3) {
-        (x < 4 ? op.img_lo : op.img_hi) |= uint64_t(img[x]) << (16 * (x & 3));
-        op.unit8 |= uint64_t(one) << (8 * x);
-      }
-    }
-    ops.push_back(op);
-  }
-  void add_poly(const PolyTerms& t) {
-    RunOp op{};
-    op.type = RUN_POLY;
-    op.k = uint32_t(t.coeffs.size());
-    op.bits = t.bits;
-    op.x = t.constant;
-    op.scalar = make_double2(t.scalar.re, t.scalar.im);
-    op.flags = (t.scalar_is_one ? 1u : 0u) | (t.root_table.empty() ? 0u : 2u);
-    op.off = uint32_t(start.size());
-    const uint32_t pbase = uint32_t(par.size());
-    for (size_t i = 0; i < t.coeffs.size(); ++i) {
-      start.push_back(pbase + (t.term_start.empty() ? 0 : t.term_start[i]));
-      coeff.push_back(t.coeffs[i]);
-      uint64_t am = 0;
-      bool single = !t.term_start.empty() && t.term_start[i + 1] > t.term_start[i];
-      for (uint32_t l = single ? t.term_start[i] : 0; single && l < t.term_start[i + 1]; ++l) {
-        single = __builtin_popcountll(t.parities[l]) == 1;
-        am |= t.parities[l];
-      }
-      and_mask.push_back(single ? am : 0);
-    }
-    start.push_back(pbase + (t.term_start.empty() ? 0 : t.term_start[t.coeffs.size()]));
-    // start[] holds nterms + 1 entries per polynomial, coeff[] and and_mask[] nterms: keep them aligned
-    coeff.push_back(0);
-    and_mask.push_back(0);
-    for (uint64_t pm : t.parities) par.push_back(pm);
-    op.toff = uint32_t(table.size());
-    for (const CplxD& c : t.root_table) table.push_back(make_double2(c.re, c.im));
-    ops.push_back(op);
-  }
-  void add_pauli(uint64_t x, uint64_t z, uint32_t ph) {
-    RunOp op{};
-    op.type = RUN_PAULI;
-    op.x = x;
-    op.z = z;
-    op.flags = ph & 3u;
-    moves |= x != 0;
-    ops.push_back(op);
-  }
-  void launch(ncsim_sparse* s) {
-    if (ops.empty()) return;
-    cudaStream_t st = s->stream;
-    if (s->m) {
-      RunOp* d_ops = upload(ops, st);
-      uint16_t* d_img = upload(image, st);
-      double2* d_ph = upload(phase, st);
-      uint8_t* d_unit = upload(unit, st);
-      double2* d_tab = upload(table, st);
-      uint32_t* d_start = upload(start, st);
-      uint64_t* d_par = upload(par, st);
-      uint64_t* d_coeff = upload(coeff, st);
-      uint64_t* d_and = upload(and_mask, st);
-      RunData d{d_ops, uint32_t(ops.size()), d_img, d_ph, d_unit, d_tab, d_start, d_par, d_coeff, d_and};
-      k_sp_run<<<sp_grid(s->m), SP_THREADS, 0, st>>>(s->key, s->amp, s->m, d);
-      NCSIM_LAUNCHED("sparse run");
-      dfree(d_ops, st);
-      dfree(d_img, st);
-      dfree(d_ph, st);
-      dfree(d_unit, st);
-      dfree(d_tab, st);
-      dfree(d_start, st);
-      dfree(d_par, st);
-      dfree(d_coeff, st);
-      dfree(d_and, st);
-    }
-    if (moves) s->sorted = false;
-    reset();
-  }
-};
 
 void sp_pauli(ncsim_sparse* s, uint64_t x, uint64_t z, uint32_t phase) {
   if (s->m) {
@@ -1218,41 +1013,15 @@ ncsim_status ncsim_sparse_run(ncsim_sparse* s, const ncsim_circuit* c, ncsim_rng
     // Paulis of sampled noise) go to the device as one pass each; a measurement, a
     // reset or a gate that creates entries ends a run
     // one builder per host thread, reused so that its tables keep their capacity across runs
-    static thread_local RunBuilder run;
+    static thread_local SlicedRun run;
     run.reset();
-    std::vector<uint32_t> img;
-    std::vector<CplxD> ph;
     for (const OpIR& op : c->ops) {
       if (op.kind == OpKind::Gate) {
-        const LoweredOp& lo = op.lowered;
-        switch (lo.kind) {
-          case LoweredKind::Nothing: continue;
-          case LoweredKind::Monomial:
-            if (lo.qubits.size() <= SP_MAX_K) {
-              run.add_mono(lo.qubits, lo.image, lo.matrix);
-              continue;
-            }
-            break;
-          case LoweredKind::PhasePoly: run.add_poly(lo.poly); continue;
-          case LoweredKind::Pauli: run.add_pauli(lo.x, lo.z, lo.phase); continue;
-          case LoweredKind::Dense:
-            if (lo.qubits.size() <= SP_MAX_K && permutation_view(lo.matrix, size_t(1) << lo.qubits.size(), img, ph)) {
-              run.add_mono(lo.qubits, img, ph);
-              continue;
-            }
-            break;
-        }
+        if (run.add_gate(op.gate, op.qubits, op.lowered)) continue;
       } else if (op.kind == OpKind::Noise) {
         // the draws do not depend on the state: a sampled error joins the run
         const int e = op.noise.sample(*rng);
-        if (e >= 0) {
-          uint64_t x = 0, z = 0;
-          for (size_t j = 0; j < op.qubits.size(); ++j) {
-            x |= uint64_t((e >> j) & 1) << op.qubits[j];
-            z |= uint64_t((e >> (8 + j)) & 1) << op.qubits[j];
-          }
-          run.add_pauli(x, z, 0);
-        }
+        if (e >= 0) run.add_pauli(op.qubits, uint64_t(e & 0xff), uint64_t(e >> 8), 0);
         continue;
       } else if (op.kind != OpKind::Measure && op.kind != OpKind::Reset) {
         continue;

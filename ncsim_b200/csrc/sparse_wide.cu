@@ -17,6 +17,7 @@
 // chunk first, orders the keys (one pass when at most 64 positions vary); a
 // gather then moves keys and amplitudes.
 #include "sparse_common.cuh"
+#include "sparse_run.hpp"
 
 using namespace ncsim;
 
@@ -133,127 +134,6 @@ __global__ void k_w_poly(const WKey<W>* key, double2* amp, uint64_t m, const __g
     const uint64_t x = local_w64(key[i], P.q, P.nq);
     poly_apply(x, amp[i], P.bits, P.nterms, P.constant, P.scalar_is_one, P.scalar, P.use_table, P.start, P.par,
                P.coeff, P.table);
-  }
-}
-
-// ---- runs of one-to-one ops in one launch ----
-enum : uint32_t { RW_MONO = 0, RW_POLY = 1, RW_PAULI = 2 };
-struct RunOpW {
-  uint32_t type;
-  uint32_t k;         // MONO: qubits; POLY: terms
-  uint16_t q[SP_MAX_K];
-  uint32_t off;       // MONO: first pattern of its tables; POLY: first term start
-  uint32_t bits;      // POLY
-  uint32_t flags;     // POLY: bit 0 scalar is one, bit 1 phasor table; PAULI: the phase
-  uint32_t toff;      // POLY: its phasor table
-  uint32_t nq, qoff;  // POLY: its qubits in RunDataW::qlist; PAULI: its masks (index into px/pz)
-  uint64_t constant;  // POLY
-  double2 scalar;     // POLY
-  // MONO on at most 3 qubits: the 8 images (16 bits each: patterns 0..3, 4..7) and unit flags
-  // (byte x: the phase of pattern x is exactly 1), packed on the host
-  uint64_t img_lo, img_hi, unit8;
-};
-struct RunDataW {
-  const RunOpW* ops;
-  uint32_t nops;
-  const uint16_t* image;
-  const double2* phase;
-  const uint8_t* unit;
-  const double2* table;
-  const uint32_t* start;
-  const uint64_t* par;
-  const uint64_t* coeff;
-  const uint16_t* qlist;
-  const void* px;  // WKey<W>[]: the runs' Pauli masks
-  const void* pz;
-};
-// One warp per block, one entry per lane.  The run's op descriptors (monomials on at most 3
-// qubits carry their image and unit tables packed into words) are staged 32 at a time into
-// shared memory, one op per lane, so the walk reads them as broadcasts instead of a chain of
-// dependent global loads per op.
-constexpr int RW_STAGE = 32;
-// One lane's key held in shared memory, word w at col[w * RW_STAGE] (consecutive lanes in
-// consecutive words: conflict-free), so the walk's bit reads and writes stay on chip.
-struct SKeyCol {
-  uint64_t* col;
-  __device__ uint32_t bit(uint32_t q) const { return uint32_t(col[(q >> 6) * RW_STAGE] >> (q & 63)) & 1u; }
-  __device__ void set(uint32_t q, uint32_t v) const {
-    uint64_t& w = col[(q >> 6) * RW_STAGE];
-    const uint64_t b = uint64_t(1) << (q & 63);
-    w = v ? (w | b) : (w & ~b);
-  }
-};
-template <int W>
-__global__ void __launch_bounds__(RW_STAGE) k_w_run(WKey<W>* key, double2* amp, uint64_t m, RunDataW d) {
-  __shared__ RunOpW s_op[RW_STAGE];
-  __shared__ uint64_t s_key[W * RW_STAGE];
-  const WKey<W>* px = static_cast<const WKey<W>*>(d.px);
-  const WKey<W>* pz = static_cast<const WKey<W>*>(d.pz);
-  const uint32_t lane = threadIdx.x;
-  const SKeyCol kk{s_key + lane};
-  for (uint64_t base = uint64_t(blockIdx.x) * RW_STAGE; base < m; base += uint64_t(gridDim.x) * RW_STAGE) {
-    const uint64_t i = base + lane;
-    const bool live = i < m;
-    double2 a = make_double2(0.0, 0.0);
-    {
-      WKey<W> k0{};
-      if (live) {
-        k0 = key[i];
-        a = amp[i];
-      }
-#pragma unroll
-      for (int w = 0; w < W; ++w) kk.col[w * RW_STAGE] = k0.w[w];
-    }
-    for (uint32_t o0 = 0; o0 < d.nops; o0 += RW_STAGE) {
-      const uint32_t cnt = min(uint32_t(RW_STAGE), d.nops - o0);
-      __syncwarp();
-      if (lane < cnt) s_op[lane] = d.ops[o0 + lane];
-      __syncwarp();
-      if (!live) continue;
-      for (uint32_t c = 0; c < cnt; ++c) {
-        const RunOpW& op = s_op[c];
-        if (op.type == RW_MONO) {
-          const uint32_t k = op.k;
-          uint32_t x = 0;
-          for (uint32_t j = 0; j < k; ++j) x |= kk.bit(op.q[j]) << j;
-          uint32_t y;
-          bool unit;
-          if (k <= 3) {
-            y = uint32_t((x < 4 ? op.img_lo : op.img_hi) >> (16 * (x & 3))) & 0xffffu;
-            unit = (op.unit8 >> (8 * x)) & 1u;
-          } else {
-            y = d.image[op.off + x];
-            unit = d.unit[op.off + x];
-          }
-          if (!unit) a = zmul(d.phase[op.off + x], a);
-          if (y != x)
-            for (uint32_t j = 0; j < k; ++j) kk.set(op.q[j], (y >> j) & 1u);
-        } else if (op.type == RW_POLY) {
-          uint64_t x = 0;
-          for (uint32_t j = 0; j < op.nq; ++j) x |= uint64_t(kk.bit(d.qlist[op.qoff + j])) << j;
-          poly_apply(x, a, op.bits, op.k, op.constant, op.flags & 1u, op.scalar, (op.flags >> 1) & 1u,
-                     d.start + op.off, d.par, d.coeff + op.off, d.table + op.toff);
-        } else {
-          const WKey<W>& zx = pz[op.qoff];
-          const WKey<W>& xx = px[op.qoff];
-          uint32_t cz = 0;
-#pragma unroll
-          for (int w = 0; w < W; ++w) {
-            cz += uint32_t(__popcll(zx.w[w] & kk.col[w * RW_STAGE]));
-            kk.col[w * RW_STAGE] ^= xx.w[w];
-          }
-          const uint32_t ph = (op.flags + 2u * cz) & 3u;
-          if (ph) a = ipow(a, ph);
-        }
-      }
-    }
-    if (live) {
-      WKey<W> k1;
-#pragma unroll
-      for (int w = 0; w < W; ++w) k1.w[w] = kk.col[w * RW_STAGE];
-      key[i] = k1;
-      amp[i] = a;
-    }
   }
 }
 
@@ -840,139 +720,16 @@ void sites_words(const PauliSites& ps, uint32_t words, std::vector<uint64_t>& x,
   phase = (ps.phase + ys) & 3u;
 }
 
-// the host side of a run of one-to-one ops
-template <int W>
-struct RunBuilderW {
-  std::vector<RunOpW> ops;
-  std::vector<uint16_t> image, qlist;
-  std::vector<double2> phase, table;
-  std::vector<uint8_t> unit;
-  std::vector<uint32_t> start;
-  std::vector<uint64_t> par, coeff;
-  std::vector<WKey<W>> px, pz;
-  bool moves = false;
-
-  void add_mono(const QubitsW& qs, const std::vector<uint32_t>& img, const std::vector<CplxD>& ph) {
-    RunOpW op{};
-    op.type = RW_MONO;
-    op.k = qs.k;
-    for (uint32_t j = 0; j < qs.k; ++j) op.q[j] = qs.q[j];
-    op.off = uint32_t(image.size());
-    for (size_t x = 0; x < img.size(); ++x) {
-      image.push_back(uint16_t(img[x]));
-      phase.push_back(make_double2(ph[x].re, ph[x].im));
-      const bool one = ph[x].re == 1.0 && ph[x].im == 0.0;
-      unit.push_back(one);
-      moves |= img[x] != x;
-      if (qs.k <= 3) {
-        (x < 4 ? op.img_lo : op.img_hi) |= uint64_t(img[x]) << (16 * (x & 3));
-        op.unit8 |= uint64_t(one) << (8 * x);
-      }
-    }
-    ops.push_back(op);
-  }
-  void add_poly(const std::vector<uint32_t>& qubits, const PolyTerms& t) {
-    check_poly_width(qubits);
-    RunOpW op{};
-    op.type = RW_POLY;
-    op.k = uint32_t(t.coeffs.size());
-    op.bits = t.bits;
-    op.constant = t.constant;
-    op.scalar = make_double2(t.scalar.re, t.scalar.im);
-    op.flags = (t.scalar_is_one ? 1u : 0u) | (t.root_table.empty() ? 0u : 2u);
-    op.nq = uint32_t(qubits.size());
-    op.qoff = uint32_t(qlist.size());
-    for (uint32_t q : qubits) qlist.push_back(uint16_t(q));
-    op.off = uint32_t(start.size());
-    const uint32_t pbase = uint32_t(par.size());
-    for (size_t i = 0; i <= t.coeffs.size(); ++i) start.push_back(pbase + (t.term_start.empty() ? 0 : t.term_start[i]));
-    for (uint64_t c : t.coeffs) coeff.push_back(c);
-    coeff.push_back(0);  // keeps coeff aligned with start (nterms + 1 per polynomial)
-    for (uint64_t pm : t.parities) par.push_back(pm);
-    op.toff = uint32_t(table.size());
-    for (const CplxD& c : t.root_table) table.push_back(make_double2(c.re, c.im));
-    ops.push_back(op);
-  }
-  void add_pauli(const uint64_t* x, const uint64_t* z, uint32_t ph) {
-    RunOpW op{};
-    op.type = RW_PAULI;
-    op.flags = ph & 3u;
-    op.qoff = uint32_t(px.size());
-    px.push_back(host_key<W>(x));
-    pz.push_back(host_key<W>(z));
-    for (int w = 0; w < W; ++w) moves |= x[w] != 0;
-    ops.push_back(op);
-  }
-  void launch(ncsim_sparse* s) {
-    if (ops.empty()) return;
-    cudaStream_t st = s->stream;
-    if (s->m) {
-      RunOpW* d_ops = upload(ops, st);
-      uint16_t* d_img = upload(image, st);
-      double2* d_ph = upload(phase, st);
-      uint8_t* d_unit = upload(unit, st);
-      double2* d_tab = upload(table, st);
-      uint32_t* d_start = upload(start, st);
-      uint64_t* d_par = upload(par, st);
-      uint64_t* d_coeff = upload(coeff, st);
-      uint16_t* d_q = upload(qlist, st);
-      WKey<W>* d_px = upload(px, st);
-      WKey<W>* d_pz = upload(pz, st);
-      RunDataW d{d_ops, uint32_t(ops.size()), d_img, d_ph, d_unit, d_tab, d_start, d_par, d_coeff, d_q, d_px, d_pz};
-      // one warp per block walks the run for 32 entries (up to 32 blocks per SM)
-      const unsigned grid =
-          unsigned(std::min<uint64_t>((s->m + RW_STAGE - 1) / RW_STAGE, uint64_t(sm_count()) * 32));
-      k_w_run<W><<<grid, RW_STAGE, 0, st>>>(keys_of<W>(s), s->amp, s->m, d);
-      NCSIM_LAUNCHED("sparse run (wide)");
-      dfree(d_ops, st);
-      dfree(d_img, st);
-      dfree(d_ph, st);
-      dfree(d_unit, st);
-      dfree(d_tab, st);
-      dfree(d_start, st);
-      dfree(d_par, st);
-      dfree(d_coeff, st);
-      dfree(d_q, st);
-      dfree(d_px, st);
-      dfree(d_pz, st);
-    }
-    if (moves) s->sorted = false;
-    *this = RunBuilderW();
-  }
-};
-
 // QuantumState::run (mod.rs:168-183) with runs of one-to-one ops in one launch each
 template <int W>
 void run_w(ncsim_sparse* s, const ncsim_circuit& c, ncsim_rng& rng, uint8_t* rec, size_t& m) {
-  RunBuilderW<W> run;
-  std::vector<uint32_t> img;
-  std::vector<CplxD> ph;
+  static thread_local SlicedRun run;  // reused, so that its buffers keep their capacity
+  run.reset();
   std::vector<uint64_t> x, z;
   for (const OpIR& op : c.ops) {
     if (op.kind == OpKind::Gate) {
       const LoweredOp& lo = op.lowered;  // on local qubits: local j is op.qubits[j]
-      switch (lo.kind) {
-        case LoweredKind::Nothing: continue;
-        case LoweredKind::Monomial:
-          if (lo.qubits.size() <= SP_MAX_K) {
-            run.add_mono(qubits_w(lo.qubits, op.qubits), lo.image, lo.matrix);
-            continue;
-          }
-          break;
-        case LoweredKind::PhasePoly:
-          run.add_poly(op.qubits, lo.poly);
-          continue;
-        case LoweredKind::Pauli:
-          embed(op.qubits, lo.x, lo.z, W, x, z);
-          run.add_pauli(x.data(), z.data(), lo.phase);
-          continue;
-        case LoweredKind::Dense:
-          if (lo.qubits.size() <= SP_MAX_K && permutation_view(lo.matrix, size_t(1) << lo.qubits.size(), img, ph)) {
-            run.add_mono(qubits_w(lo.qubits, op.qubits), img, ph);
-            continue;
-          }
-          break;
-      }
+      if (run.add_gate(op.gate, op.qubits, lo)) continue;
       run.launch(s);
       apply_lowered_w<W>(s, lo, op.qubits);
       continue;
@@ -980,16 +737,7 @@ void run_w(ncsim_sparse* s, const ncsim_circuit& c, ncsim_rng& rng, uint8_t* rec
     if (op.kind == OpKind::Noise) {
       // Noise::sample (circuit.rs:136-146): the draws do not depend on the state
       const int e = op.noise.sample(rng);
-      if (e >= 0) {
-        x.assign(W, 0);
-        z.assign(W, 0);
-        for (size_t j = 0; j < op.qubits.size(); ++j) {
-          const uint32_t q = op.qubits[j];
-          x[q >> 6] |= uint64_t((e >> j) & 1) << (q & 63);
-          z[q >> 6] |= uint64_t((e >> (8 + j)) & 1) << (q & 63);
-        }
-        run.add_pauli(x.data(), z.data(), 0);
-      }
+      if (e >= 0) run.add_pauli(op.qubits, uint64_t(e & 0xff), uint64_t(e >> 8), 0);
       continue;
     }
     if (op.kind == OpKind::Measure) {
