@@ -27,6 +27,7 @@ SOURCES = [
     "csrc/sparse.cu",
     "csrc/sparse_wide.cu",
     "csrc/sparse_run.cu",
+    "csrc/sparse_dense.cu",
     "csrc/frames.cu",
     "csrc/frames_plan.cpp",
     "csrc/host/ir.cpp",
@@ -39,6 +40,7 @@ HEADERS = [
     "csrc/engine.cuh",
     "csrc/sparse_common.cuh",
     "csrc/sparse_run.hpp",
+    "csrc/sparse_dense.hpp",
     "csrc/host_math.hpp",
     "csrc/fused_plan.hpp",
     "csrc/batch_plan.hpp",

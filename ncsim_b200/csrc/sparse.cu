@@ -13,6 +13,7 @@
 // added on the host in a fixed order; Born sampling takes the cumulative
 // weights in entry order on the host, as sparse.rs:407-424 does.
 #include "sparse_common.cuh"
+#include "sparse_dense.hpp"
 #include "sparse_run.hpp"
 
 using namespace ncsim;
@@ -513,7 +514,12 @@ void sp_phasepoly(ncsim_sparse* s, const PolyTerms& t) {
 void sp_apply_lowered(ncsim_sparse* s, const LoweredOp& op) {
   switch (op.kind) {
     case LoweredKind::Nothing: return;
-    case LoweredKind::Dense: sp_matrix(s, op.qubits, op.matrix); return;
+    case LoweredKind::Dense: {
+      SparseDense1 d;
+      if (sparse_dense1(op, op.qubits, d)) sparse_apply_dense1(s, {d});
+      else sp_matrix(s, op.qubits, op.matrix);
+      return;
+    }
     case LoweredKind::Monomial: sp_monomial(s, op.qubits, op.image, op.matrix); return;
     case LoweredKind::PhasePoly: sp_phasepoly(s, op.poly); return;
     case LoweredKind::Pauli: sp_pauli(s, op.x, op.z, op.phase); return;
@@ -641,6 +647,10 @@ void check_words(const ncsim_sparse* s, uint32_t words, std::initializer_list<co
 }
 
 }  // namespace
+
+namespace ncsim {
+void sparse_sort(ncsim_sparse* s) { sp_sort(s); }
+}  // namespace ncsim
 
 extern "C" {
 
@@ -1015,7 +1025,18 @@ ncsim_status ncsim_sparse_run(ncsim_sparse* s, const ncsim_circuit* c, ncsim_rng
     // one builder per host thread, reused so that its tables keep their capacity across runs
     static thread_local SlicedRun run;
     run.reset();
+    std::vector<SparseDense1> dense;  // consecutive dense 1-qubit gates
+    SparseDense1 d;
     for (const OpIR& op : c->ops) {
+      if (op.kind == OpKind::Gate && sparse_dense1(op.lowered, op.qubits, d)) {
+        run.launch(s);
+        dense.push_back(d);
+        continue;
+      }
+      if (op.kind == OpKind::Gate || op.kind == OpKind::Noise || op.kind == OpKind::Measure || op.kind == OpKind::Reset) {
+        sparse_apply_dense1(s, dense);
+        dense.clear();
+      }
       if (op.kind == OpKind::Gate) {
         if (run.add_gate(op.gate, op.qubits, op.lowered)) continue;
       } else if (op.kind == OpKind::Noise) {
@@ -1031,6 +1052,7 @@ ncsim_status ncsim_sparse_run(ncsim_sparse* s, const ncsim_circuit* c, ncsim_rng
       if (r >= 0) rec[m++] = uint8_t(r);
     }
     run.launch(s);
+    sparse_apply_dense1(s, dense);
     NCSIM_CUDA(cudaStreamSynchronize(s->stream));
     if (len) *len = m;
   });

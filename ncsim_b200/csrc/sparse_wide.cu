@@ -17,6 +17,7 @@
 // chunk first, orders the keys (one pass when at most 64 positions vary); a
 // gather then moves keys and amplitudes.
 #include "sparse_common.cuh"
+#include "sparse_dense.hpp"
 #include "sparse_run.hpp"
 
 using namespace ncsim;
@@ -634,7 +635,11 @@ template <int W>
 void apply_lowered_w(ncsim_sparse* s, const LoweredOp& lo, const std::vector<uint32_t>& qubits) {
   switch (lo.kind) {
     case LoweredKind::Nothing: return;
-    case LoweredKind::Dense: return matrix_w<W>(s, qubits_w(lo.qubits, qubits), lo.matrix);
+    case LoweredKind::Dense: {
+      SparseDense1 d;
+      if (sparse_dense1(lo, qubits, d)) return sparse_apply_dense1(s, {d});
+      return matrix_w<W>(s, qubits_w(lo.qubits, qubits), lo.matrix);
+    }
     case LoweredKind::Monomial: return monomial_w<W>(s, qubits_w(lo.qubits, qubits), lo.image, lo.matrix);
     case LoweredKind::PhasePoly: return poly_w<W>(s, qubits, lo.poly);
     case LoweredKind::Pauli: {
@@ -726,7 +731,18 @@ void run_w(ncsim_sparse* s, const ncsim_circuit& c, ncsim_rng& rng, uint8_t* rec
   static thread_local SlicedRun run;  // reused, so that its buffers keep their capacity
   run.reset();
   std::vector<uint64_t> x, z;
+  std::vector<SparseDense1> dense;  // consecutive dense 1-qubit gates
+  SparseDense1 d;
   for (const OpIR& op : c.ops) {
+    if (op.kind == OpKind::Gate && sparse_dense1(op.lowered, op.qubits, d)) {
+      run.launch(s);
+      dense.push_back(d);
+      continue;
+    }
+    if (op.kind == OpKind::Gate || op.kind == OpKind::Noise || op.kind == OpKind::Measure || op.kind == OpKind::Reset) {
+      sparse_apply_dense1(s, dense);
+      dense.clear();
+    }
     if (op.kind == OpKind::Gate) {
       const LoweredOp& lo = op.lowered;  // on local qubits: local j is op.qubits[j]
       if (run.add_gate(op.gate, op.qubits, lo)) continue;
@@ -762,6 +778,7 @@ void run_w(ncsim_sparse* s, const ncsim_circuit& c, ncsim_rng& rng, uint8_t* rec
     }
   }
   run.launch(s);
+  sparse_apply_dense1(s, dense);
 }
 
 }  // namespace
