@@ -57,6 +57,8 @@ std::mutex g_pool_mu;
 cudaMemPool_t g_pool[POOL_DEVICES] = {};
 }  // namespace
 
+void sparse_trim();  // the sparse form's kept streams and buffers (sparse.cu)
+
 cudaMemPool_t lib_pool() {
   int dev = 0;
   NCSIM_CUDA(cudaGetDevice(&dev));
@@ -377,7 +379,10 @@ ncsim_status ncsim_device_info(int32_t* sm, uint64_t* free_b, uint64_t* total_b)
 }
 
 ncsim_status ncsim_trim_memory(void) {
-  return guarded([&] { trim_lib_pools(); });
+  return guarded([&] {
+    sparse_trim();
+    trim_lib_pools();
+  });
 }
 
 ncsim_status ncsim_pool_info(uint64_t* reserved_bytes, uint64_t* used_bytes) {

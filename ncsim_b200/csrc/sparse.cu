@@ -12,6 +12,8 @@
 // Sums over entries (norm, expectation, inner product) are FP64 block partials
 // added on the host in a fixed order; Born sampling takes the cumulative
 // weights in entry order on the host, as sparse.rs:407-424 does.
+#include <map>
+
 #include "sparse_common.cuh"
 #include "sparse_dense.hpp"
 #include "sparse_run.hpp"
@@ -585,31 +587,82 @@ int sp_apply_op(ncsim_sparse* s, const OpIR& op, ncsim_rng& rng) {
   }
 }
 
+// What a state needs beside its entries: a stream, the reduction partials and their pinned mirror.
+// A released state's set is kept for the next state of the device (making and freeing one takes
+// about as long as a short circuit: the pinned allocation and cudaFree, which waits for the whole
+// device).  At most KEPT_SETS are kept per device; ncsim_trim_memory gives them back.
+struct SpSet {
+  cudaStream_t stream = nullptr;
+  double* partials = nullptr;
+  double* host_partials = nullptr;
+};
+constexpr size_t KEPT_SETS = 8;
+std::mutex& kept_mu() {
+  static std::mutex* m = new std::mutex;  // outlives every state
+  return *m;
+}
+std::map<int, std::vector<SpSet>>& kept_sets() {
+  static auto* m = new std::map<int, std::vector<SpSet>>;
+  return *m;
+}
+void free_set(SpSet& r) {
+  cudaFree(r.partials);
+  cudaFreeHost(r.host_partials);
+  if (r.stream) cudaStreamDestroy(r.stream);
+}
+
 ncsim_sparse* sp_new(uint32_t n) {
   const uint32_t words = spw::words_for(n);  // checks 1 <= n <= 1024
   auto s = std::make_unique<ncsim_sparse>();
   s->n = n;
   s->words = words;
   NCSIM_CUDA(cudaGetDevice(&s->device));
-  NCSIM_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
-  NCSIM_CUDA(cudaMalloc(&s->partials, SP_BLOCKS * 2 * sizeof(double)));
-  NCSIM_CUDA(cudaMallocHost(&s->host_partials, SP_BLOCKS * 2 * sizeof(double)));
-  NCSIM_CUDA(cudaEventCreate(&s->timer0));
-  NCSIM_CUDA(cudaEventCreate(&s->timer1));
+  {
+    std::lock_guard<std::mutex> lk(kept_mu());
+    auto& kept = kept_sets()[s->device];
+    if (!kept.empty()) {
+      s->stream = kept.back().stream;
+      s->partials = kept.back().partials;
+      s->host_partials = kept.back().host_partials;
+      kept.pop_back();
+      return s.release();
+    }
+  }
+  SpSet r;
+  try {
+    NCSIM_CUDA(cudaStreamCreateWithFlags(&r.stream, cudaStreamNonBlocking));
+    NCSIM_CUDA(cudaMalloc(&r.partials, SP_BLOCKS * 2 * sizeof(double)));
+    NCSIM_CUDA(cudaMallocHost(&r.host_partials, SP_BLOCKS * 2 * sizeof(double)));
+  } catch (...) {
+    free_set(r);
+    throw;
+  }
+  s->stream = r.stream;
+  s->partials = r.partials;
+  s->host_partials = r.host_partials;
   return s.release();
 }
 
 void sp_release(ncsim_sparse* s) {
   if (!s) return;
   cudaSetDevice(s->device);
-  if (s->stream) cudaStreamSynchronize(s->stream);
-  cudaFree(s->key);
-  cudaFree(s->amp);
-  cudaFree(s->partials);
-  cudaFreeHost(s->host_partials);
+  dfree(s->key, s->stream);
+  dfree(s->amp, s->stream);
+  SpSet r;
+  r.stream = s->stream;
+  r.partials = s->partials;
+  r.host_partials = s->host_partials;
+  const bool idle = cudaStreamSynchronize(s->stream) == cudaSuccess;  // a set is kept with nothing queued on it
   if (s->timer0) cudaEventDestroy(s->timer0);
   if (s->timer1) cudaEventDestroy(s->timer1);
-  if (s->stream) cudaStreamDestroy(s->stream);
+  bool keep = false;
+  if (idle) {
+    std::lock_guard<std::mutex> lk(kept_mu());
+    auto& kept = kept_sets()[s->device];
+    keep = kept.size() < KEPT_SETS;
+    if (keep) kept.push_back(r);
+  }
+  if (!keep) free_set(r);
   delete s;
 }
 
@@ -650,6 +703,20 @@ void check_words(const ncsim_sparse* s, uint32_t words, std::initializer_list<co
 
 namespace ncsim {
 void sparse_sort(ncsim_sparse* s) { sp_sort(s); }
+void sparse_trim() {
+  std::map<int, std::vector<SpSet>> sets;
+  {
+    std::lock_guard<std::mutex> lk(kept_mu());
+    sets.swap(kept_sets());
+  }
+  int cur = 0;
+  cudaGetDevice(&cur);
+  for (auto& kv : sets) {
+    cudaSetDevice(kv.first);
+    for (SpSet& r : kv.second) free_set(r);
+  }
+  cudaSetDevice(cur);
+}
 }  // namespace ncsim
 
 extern "C" {
@@ -1158,6 +1225,7 @@ ncsim_status ncsim_sparse_timer_start(ncsim_sparse* s) {
   return guarded([&] {
     need(s, "state");
     Lock lk(s);
+    if (!s->timer0) NCSIM_CUDA(cudaEventCreate(&s->timer0));
     NCSIM_CUDA(cudaEventRecord(s->timer0, s->stream));
   });
 }
@@ -1167,6 +1235,8 @@ ncsim_status ncsim_sparse_timer_stop(ncsim_sparse* s, double* milliseconds) {
     need(s, "state");
     need(milliseconds, "out");
     Lock lk(s);
+    if (!s->timer0) throw Error(NCSIM_ERR_DEVICE, "timer stopped before it was started");
+    if (!s->timer1) NCSIM_CUDA(cudaEventCreate(&s->timer1));
     NCSIM_CUDA(cudaEventRecord(s->timer1, s->stream));
     NCSIM_CUDA(cudaEventSynchronize(s->timer1));
     float ms = 0;
