@@ -202,6 +202,8 @@ CplxD state_norm_sq(const ncsim_state* s) {
   return {v, 0.0};
 }
 
+void check_pauli_on(const ncsim_state* s, uint64_t x, uint64_t z) { check_pauli(s, x, z); }
+
 CplxD state_expectation(const ncsim_state* s, uint64_t x, uint64_t z, uint32_t phase) {
   check_pauli(s, x, z);
   double v[2];

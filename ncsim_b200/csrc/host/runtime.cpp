@@ -15,6 +15,8 @@ namespace ncsim {
 
 PolyTerms build_poly_terms(const PhasePolyIR& p, const std::vector<uint32_t>& qubits, const Phase& scalar);
 
+void state_expectations(const ncsim_state* s, uint64_t count, const uint64_t* x, const uint64_t* z, const uint32_t* phase,
+                        CplxD* out);
 struct PlainPlan;
 std::shared_ptr<PlainPlan> plan_plain_passes(uint32_t n, int precision, const std::vector<const LoweredOp*>& gates);
 void run_plain_plan(ncsim_state* s, PlainPlan& P);
@@ -527,8 +529,10 @@ ncsim_status ncsim_sv_expectation_sum(const ncsim_state* s, uint64_t count, cons
     }
     std::lock_guard<std::recursive_mutex> lk(s->mu);
     std::vector<CplxD> t(count);
+    std::vector<CplxD> es(count);
+    state_expectations(s, count, x, z, phase, es.data());
     for (uint64_t k = 0; k < count; ++k) {
-      CplxD e = state_expectation(s, x[k], z[k], phase[k] & 3);
+      const CplxD e = es[k];
       const double cr = coeffs[2 * k], ci = coeffs[2 * k + 1];
       t[k] = {cr * e.re - ci * e.im, cr * e.im + ci * e.re};
     }
