@@ -299,51 +299,51 @@ void state_gather(const ncsim_state* s, const uint64_t* idx, uint64_t count, dou
   NCSIM_CUDA(cudaStreamSynchronize(s->stream));
 }
 
-// StateVector::sample (vector.rs:494-540): block weights on the device, the
-// block of every shot on the host (the reference's sequential running sum),
-// the walk inside the block on the device.
+// StateVector::sample (vector.rs:494-540): block weights on the device, their running sum on
+// the host (the reference's sequential one), every shot's block and walk on the device.
 void state_sample(const ncsim_state* s, const double* uniforms, uint64_t shots, uint64_t* out) {
   const uint64_t block = std::min<uint64_t>(4096, s->len);
   const uint64_t nblocks = s->len / block;
-  std::vector<double> w(nblocks);
-  double* d_w = nullptr;
-  NCSIM_CUDA(pool_alloc(&d_w, nblocks * sizeof(double), s->stream));
-  launch_block_weights(s, d_w, nblocks, block);
-  NCSIM_CUDA(cudaMemcpyAsync(w.data(), d_w, nblocks * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-  NCSIM_CUDA(cudaFreeAsync(d_w, s->stream));
-  NCSIM_CUDA(cudaStreamSynchronize(s->stream));
   std::vector<double> hi(nblocks);
+  // what a call takes from the pool, given back in stream order on every way out
+  struct Buffers {
+    cudaStream_t st;
+    double *w = nullptr, *ends = nullptr, *u = nullptr;
+    uint64_t* out = nullptr;
+    ~Buffers() {
+      for (void* p : {(void*)w, (void*)ends, (void*)u, (void*)out})
+        if (p) cudaFreeAsync(p, st);
+    }
+  } d{s->stream};
+  NCSIM_CUDA(pool_alloc(&d.w, nblocks * sizeof(double), s->stream));
+  launch_block_weights(s, d.w, nblocks, block);
+  NCSIM_CUDA(cudaMemcpyAsync(hi.data(), d.w, nblocks * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+  NCSIM_CUDA(cudaStreamSynchronize(s->stream));
   double total = 0.0;
   for (uint64_t b = 0; b < nblocks; ++b) {
-    total += w[b];
+    total += hi[b];
     hi[b] = total;
   }
   if (!(total > 0.0)) throw Error(NCSIM_ERR_ZERO_STATE, "state vanished: sample");
   if (shots == 0) return;
   need(uniforms, "uniforms");
   need(out, "output");
-  std::vector<double> u(shots), acc(shots);
-  std::vector<uint64_t> blk(shots);
-  for (uint64_t k = 0; k < shots; ++k) {
-    u[k] = uniforms[k] * total;
-    // the first block whose running sum exceeds u, else the last block
-    uint64_t b = uint64_t(std::upper_bound(hi.begin(), hi.end(), u[k]) - hi.begin());
-    if (b >= nblocks) b = nblocks - 1;
-    blk[k] = b;
-    acc[k] = b ? hi[b - 1] : 0.0;
+  NCSIM_CUDA(pool_alloc(&d.u, shots * sizeof(double), s->stream));
+  NCSIM_CUDA(pool_alloc(&d.out, shots * sizeof(uint64_t), s->stream));
+  NCSIM_CUDA(cudaMemcpyAsync(d.w, hi.data(), nblocks * sizeof(double), cudaMemcpyHostToDevice, s->stream));
+  NCSIM_CUDA(cudaMemcpyAsync(d.u, uniforms, shots * sizeof(double), cudaMemcpyHostToDevice, s->stream));
+  // The parts read the register once more, a walk half a block per shot: they pay from about a shot
+  // per block on (1/128 of a complex128 register's bytes; without room for them the shots walk).
+  if (block == 4096 && shots >= nblocks) {
+    if (pool_alloc(&d.ends, nblocks * 32 * sizeof(double), s->stream) == cudaSuccess) {
+      launch_sample_parts(s, d.w, nblocks, block, d.ends);
+    } else {
+      cudaGetLastError();
+      d.ends = nullptr;
+    }
   }
-  double *d_u = nullptr, *d_acc = nullptr;
-  uint64_t *d_blk = nullptr, *d_out = nullptr;
-  NCSIM_CUDA(pool_alloc(&d_u, shots * sizeof(double), s->stream));
-  NCSIM_CUDA(pool_alloc(&d_acc, shots * sizeof(double), s->stream));
-  NCSIM_CUDA(pool_alloc(&d_blk, shots * sizeof(uint64_t), s->stream));
-  NCSIM_CUDA(pool_alloc(&d_out, shots * sizeof(uint64_t), s->stream));
-  NCSIM_CUDA(cudaMemcpyAsync(d_u, u.data(), shots * sizeof(double), cudaMemcpyHostToDevice, s->stream));
-  NCSIM_CUDA(cudaMemcpyAsync(d_acc, acc.data(), shots * sizeof(double), cudaMemcpyHostToDevice, s->stream));
-  NCSIM_CUDA(cudaMemcpyAsync(d_blk, blk.data(), shots * sizeof(uint64_t), cudaMemcpyHostToDevice, s->stream));
-  launch_sample_walk(s, d_u, d_blk, d_acc, shots, block, d_out);
-  NCSIM_CUDA(cudaMemcpyAsync(out, d_out, shots * sizeof(uint64_t), cudaMemcpyDeviceToHost, s->stream));
-  for (void* p : {(void*)d_u, (void*)d_acc, (void*)d_blk, (void*)d_out}) NCSIM_CUDA(cudaFreeAsync(p, s->stream));
+  launch_sample_find(s, d.u, total, d.w, nblocks, d.ends, shots, block, d.out);
+  NCSIM_CUDA(cudaMemcpyAsync(out, d.out, shots * sizeof(uint64_t), cudaMemcpyDeviceToHost, s->stream));
   NCSIM_CUDA(cudaStreamSynchronize(s->stream));
 }
 

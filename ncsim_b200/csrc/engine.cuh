@@ -314,6 +314,9 @@ int launch_project_partials(ncsim_state* s, uint64_t x, uint64_t z, uint32_t pha
 int launch_compare_partials(const ncsim_state* a, const ncsim_state* b, double* maxdiff_dev);
 // sampling
 void launch_block_weights(const ncsim_state* s, double* weights_dev, uint64_t nblocks, uint64_t block);
+void launch_sample_parts(const ncsim_state* s, const double* hi_dev, uint64_t nblocks, uint64_t block, double* ends_dev);
+void launch_sample_find(const ncsim_state* s, const double* uniforms_dev, double total, const double* hi_dev, uint64_t nblocks,
+                        const double* ends_dev, uint64_t shots, uint64_t block, uint64_t* out_dev);
 void launch_sample_walk(const ncsim_state* s, const double* u_dev, const uint64_t* blk_dev, const double* acc_dev,
                         uint64_t shots, uint64_t block, uint64_t* out_dev);
 
