@@ -313,6 +313,17 @@ int launch_project_partials(ncsim_state* s, uint64_t x, uint64_t z, uint32_t pha
 // slots: <a|b> re, im, <a|a>, <b|b>; the per-block max |a-b| goes to maxdiff_dev[block]
 int launch_compare_partials(const ncsim_state* a, const ncsim_state* b, double* maxdiff_dev);
 // sampling
+// Measurements of a run decided on the device: the uniforms that they may need, drawn ahead in stream order
+// (an uncertain outcome takes the next one), and the outcomes.
+constexpr int MEASURE_QUEUE = 256;
+struct MeasureQueue {
+  double uniform[MEASURE_QUEUE];
+  int outcome[MEASURE_QUEUE];
+  uint32_t used;    // uniforms taken
+  uint32_t ticket;  // blocks of the current reduction that have stored their partial
+};
+bool can_measure_on_device(const ncsim_state* s);
+void launch_measure(ncsim_state* s, uint64_t x, uint64_t z, uint32_t phase, MeasureQueue* queue, int slot, bool reset);
 void launch_block_weights(const ncsim_state* s, double* weights_dev, uint64_t nblocks, uint64_t block);
 void launch_sample_parts(const ncsim_state* s, const double* hi_dev, uint64_t nblocks, uint64_t block, double* ends_dev);
 void launch_sample_find(const ncsim_state* s, const double* uniforms_dev, double total, const double* hi_dev, uint64_t nblocks,

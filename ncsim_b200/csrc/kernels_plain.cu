@@ -600,6 +600,20 @@ __global__ void __launch_bounds__(THREADS) k_pauli_pair(V<R>* __restrict__ a, ui
   }
 }
 
+// X on bit h when the measurement before it came out 1 (a reset's flip)
+template <class R>
+__global__ void __launch_bounds__(THREADS) k_flip_if(V<R>* __restrict__ a, uint64_t npairs, int h, const int* decided) {
+  if (!*decided) return;
+  const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+  const uint64_t lo = (uint64_t(1) << h) - 1;
+  for (uint64_t p = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < npairs; p += stride) {
+    const uint64_t c = ((p & ~lo) << 1) | (p & lo), d = c | (lo + 1);
+    const V<R> vc = a[c];
+    a[c] = a[d];
+    a[d] = vc;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // elementwise
 // ---------------------------------------------------------------------------
@@ -718,10 +732,50 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_norm(const V<R>* __restrict_
   block_store<1>(acc, partials);
 }
 
-// <psi|P|psi> (and optionally <psi|psi>): slots re, im[, norm]
+// A measurement decided on the device (QuantumState::measure, mod.rs:113-131): the last block of the
+// reduction sums the partials in fetch_partials' order and takes the outcome by the host's rule, with the
+// next of the uniforms drawn ahead when it is uncertain.
+constexpr int DECIDE_BLOCKS = 1024;  // reductions of at most this many blocks
+__device__ void decide_in_last_block(const double* partials, MeasureQueue* q, int slot) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {  // the thread that stored this block's partial
+    __threadfence();
+    last = atomicAdd(&q->ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __shared__ double v[2][DECIDE_BLOCKS];
+  const int nb = int(gridDim.x);
+  for (int i = threadIdx.x; i < nb; i += blockDim.x) {
+    v[0][i] = __ldcg(partials + i * PARTIAL_SLOTS);      // <P>, its real part
+    v[1][i] = __ldcg(partials + i * PARTIAL_SLOTS + 2);  // <psi|psi>
+  }
+  __syncthreads();
+  for (int m = nb; m > 1;) {
+    const int h = (m + 1) / 2;
+    for (int i = threadIdx.x; i + h < m; i += blockDim.x) {
+      v[0][i] = __dadd_rn(v[0][i], v[0][i + h]);
+      v[1][i] = __dadd_rn(v[1][i], v[1][i + h]);
+    }
+    __syncthreads();
+    m = h;
+  }
+  if (threadIdx.x == 0) {
+    double p = __dadd_rn(1.0, __ddiv_rn(v[0][0], v[1][0])) * 0.5;
+    if (!isnan(p)) p = fmin(1.0, fmax(0.0, p));
+    int outcome;
+    if (p > 1.0 - 1e-12) outcome = 0;
+    else if (p < 1e-12) outcome = 1;
+    else outcome = q->uniform[q->used++] >= p;
+    q->outcome[slot] = outcome;
+    q->ticket = 0;
+  }
+}
+
+// <psi|P|psi> (and optionally <psi|psi>): slots re, im[, norm]; with a queue the measurement's outcome too
 template <class R, bool NORM>
 __global__ void __launch_bounds__(REDUCE_THREADS) k_expect_diag(const V<R>* __restrict__ a, uint64_t len, uint64_t z, int ph,
-                                                                double* partials) {
+                                                                double* partials, MeasureQueue* queue = nullptr, int slot = 0) {
   // sum_c i^{k(c)} |psi(c)|^2
   double acc[3] = {0.0, 0.0, 0.0};
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
@@ -741,11 +795,13 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_expect_diag(const V<R>* __re
     }
   }
   block_store<3>(acc, partials);
+  if (NORM && queue) decide_in_last_block(partials, queue, slot);
 }
 
 template <class R, bool NORM>
 __global__ void __launch_bounds__(REDUCE_THREADS) k_expect_pair(const V<R>* __restrict__ a, uint64_t npairs, int h, uint64_t x,
-                                                                uint64_t z, int ph, double* partials) {
+                                                                uint64_t z, int ph, double* partials,
+                                                                MeasureQueue* queue = nullptr, int slot = 0) {
   double acc[3] = {0.0, 0.0, 0.0};
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   const uint64_t lo = (uint64_t(1) << h) - 1;
@@ -776,6 +832,7 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_expect_pair(const V<R>* __re
     }
   }
   block_store<3>(acc, partials);
+  if (NORM && queue) decide_in_last_block(partials, queue, slot);
 }
 
 template <class R>
@@ -832,7 +889,8 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_compare(const V<RA>* __restr
 // projection (1 + s P)/2 fused with the norm of the result
 template <class R>
 __global__ void __launch_bounds__(REDUCE_THREADS) k_project_diag(V<R>* __restrict__ a, uint64_t len, uint64_t z, int ph, int outcome,
-                                                                 double* partials) {
+                                                                 double* partials, const int* decided = nullptr) {
+  if (decided) outcome = *decided;  // a measurement's, taken on the device
   double acc[1] = {0.0};
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   for (uint64_t c0 = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; c0 < len; c0 += UNROLL * stride) {
@@ -856,7 +914,9 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_project_diag(V<R>* __restric
 
 template <class R>
 __global__ void __launch_bounds__(REDUCE_THREADS) k_project_pair(V<R>* __restrict__ a, uint64_t npairs, int h, uint64_t x, uint64_t z,
-                                                                 int ph, int outcome, double* partials) {
+                                                                 int ph, int outcome, double* partials,
+                                                                 const int* decided = nullptr) {
+  if (decided) outcome = *decided;
   double acc[1] = {0.0};
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   const uint64_t lo = (uint64_t(1) << h) - 1;
@@ -1524,6 +1584,41 @@ int launch_project_partials(ncsim_state* s, uint64_t x, uint64_t z, uint32_t pha
   });
   NCSIM_LAUNCHED("project");
   return g;
+}
+
+bool can_measure_on_device(const ncsim_state* s) { return reduce_grid(s->len) <= DECIDE_BLOCKS; }
+
+// measurement `slot` of the queue: outcome and projection, nothing waited for; a reset also flips on 1
+void launch_measure(ncsim_state* s, uint64_t x, uint64_t z, uint32_t phase, MeasureQueue* queue, int slot, bool reset) {
+  const int ph = int(phase & 3);
+  const int* decided = &queue->outcome[slot];
+  NCSIM_DISPATCH(s, {
+    if (x == 0) {
+      const int g = reduce_grid(s->len);
+      {
+        ProfScope ps(s, K_EXPECT, 0.5 * full_bytes(s));
+        k_expect_diag<R, true><<<g, REDUCE_THREADS, 0, s->stream>>>(amp_of<R>(s), s->len, z, ph, s->partials, queue, slot);
+      }
+      ProfScope ps(s, K_PROJECT, 0.5 * full_bytes(s));
+      k_project_diag<R><<<g, REDUCE_THREADS, 0, s->stream>>>(amp_of<R>(s), s->len, z, ph, 0, s->partials, decided);
+    } else {
+      const int h = 63 - __builtin_clzll(x);
+      const uint64_t np = s->len >> 1;
+      const int g = reduce_grid(np);
+      {
+        ProfScope ps(s, K_EXPECT, 0.5 * full_bytes(s));
+        k_expect_pair<R, true><<<g, REDUCE_THREADS, 0, s->stream>>>(amp_of<R>(s), np, h, x, z, ph, s->partials, queue, slot);
+      }
+      ProfScope ps(s, K_PROJECT, full_bytes(s));
+      k_project_pair<R><<<g, REDUCE_THREADS, 0, s->stream>>>(amp_of<R>(s), np, h, x, z, ph, 0, s->partials, decided);
+    }
+    if (reset) {
+      ProfScope ps(s, K_PAULI, full_bytes(s));
+      const uint64_t np = s->len >> 1;
+      k_flip_if<R><<<grid_for(np, THREADS), THREADS, 0, s->stream>>>(amp_of<R>(s), np, 63 - __builtin_clzll(z), decided);
+    }
+  });
+  NCSIM_LAUNCHED("measure");
 }
 
 void launch_block_weights(const ncsim_state* s, double* w, uint64_t nblocks, uint64_t block) {
