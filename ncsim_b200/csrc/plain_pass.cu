@@ -22,8 +22,12 @@
 // What bounds a pass: instruction issue and its latency (random layers at n = 24,
 // ncu: issue slots 47% busy, FP64 pipe 27%, shared memory 29%, DRAM 18%), not HBM.
 // Measured on random layers of depth 20, complex128, against 8-amplitude cubes on
-// 4096-amplitude tiles (one 512-thread CTA per SM): n = 20 0.80 -> 0.49 ms, n = 24
-// 11.8 -> 5.3 ms, n = 28 221 -> 100 ms.
+// 4096-amplitude tiles (one 512-thread CTA per SM): n = 20 0.80 -> 0.44 ms, n = 24
+// 11.8 -> 4.9 ms, n = 28 221 -> 93 ms.  An op that does nothing costs about 50
+// instructions, so signs that follow one another (a layer's CZs) are one op with a list
+// (n = 28 100 -> 96 ms) and a skipped op goes through the dispatch's empty case instead of
+// a branch around it (96 -> 93 ms).  Storing the last chain's cubes straight to the
+// register instead of through the tile was slower (96 ms).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -94,7 +98,7 @@ enum DevKind : uint32_t {
   DK_TURN,                           // + j: quarter turn (+-i) on the half with bit j set: parts exchanged, one negated
   DK_TURN_ALL = DK_TURN + CUBE_BITS,
   DK_TURN_MASK,
-  DK_SIGN,                           // sign of the cube elements of a mask, kept pending in a bit mask
+  DK_SIGNS,                          // signs of cube elements, kept pending in a bit mask: em items from item gml on
   DK_FLUSH,                          // the pending signs applied
   DK_RZ,                             // + j: two phases selected by cube bit j
   DK_RZ_OUT = DK_RZ + CUBE_BITS,     // two phases selected by a tile bit outside the cube
@@ -132,6 +136,12 @@ struct OpHead {
   uint32_t kind;
   uint32_t em;        // cube elements (bit b: element b); chain: number of ops
   uint32_t gml, gvl;  // fixed tile bits outside the cube, and their values; chain: cube bits, chain number
+};
+// One sign: the cube elements em of the threads and tiles whose fixed bits are all one.
+struct SignItem {
+  uint32_t fix;   // tile bits outside the cube
+  uint32_t em;
+  uint64_t gfix;  // bits outside the window
 };
 struct OpCond {
   uint64_t gfix, gval;  // fixed bits outside the window, and the values the tile base must have there
@@ -211,7 +221,8 @@ struct PassParams {
   const V<R>* cpool;
   const uint32_t* upool;
   const uint64_t* ppool;  // phase polynomial parities (global masks)
-  uint32_t nchains;
+  uint32_t nchains, nsigns;
+  SignItem sign[MAX_PASS_OPS];   // copied into shared memory once per CTA, like the arguments
   OpHead head[MAX_PASS_OPS];
   OpCond cond[MAX_PASS_OPS];
   OpArgs<R> args[MAX_PASS_OPS];  // copied into shared memory once per CTA
@@ -480,7 +491,7 @@ __device__ __forceinline__ V<R> table_elem(V<R> v, uint32_t e, uint32_t xout, co
 // spread over the tile bits outside the cube).
 template <class R>
 __device__ __forceinline__ void tile_chain(uint32_t tile, uint32_t o, uint32_t gbase, const OpArgs<R>* args,
-                                           const PassParams<R>& P, uint64_t base) {
+                                           const SignItem* signs, const PassParams<R>& P, uint64_t base) {
   V<R>* const t = shared_tile<R>() + tile;  // an index into the shared array, so that accesses stay in the shared space
   const uint32_t nsub = P.head[o].em;
   const uint32_t cbits = P.head[o].gml;  // cube bit j: byte j
@@ -502,12 +513,10 @@ __device__ __forceinline__ void tile_chain(uint32_t tile, uint32_t o, uint32_t g
     v[b] = t[sg ^ a];
   }
   uint32_t pend = 0;  // elements whose sign is still to be flipped
-  OpHead hn = P.head[o + 1];
   for (uint32_t s = o + 1; s <= o + nsub; ++s) {
-    const OpHead h = hn;
-    hn = P.head[min(s + 1, uint32_t(MAX_PASS_OPS - 1))];  // in flight while this op runs
+    const OpHead h = P.head[s];
     const OpArgs<R>& op = args[s];
-    if ((h.kind & DK_COND) && (base & P.cond[s].gfix) != P.cond[s].gval) continue;  // uniform over the CTA
+    const bool skip = (h.kind & DK_COND) && (base & P.cond[s].gfix) != P.cond[s].gval;  // uniform over the CTA
     const bool on = (gb & h.gml) == h.gvl;
     const uint32_t em = h.em;
 #define NCSIM_D1(j) \
@@ -524,7 +533,7 @@ __device__ __forceinline__ void tile_chain(uint32_t tile, uint32_t o, uint32_t g
 #define NCSIM_SW(i, X) \
   case DK_SWAP + i: if (on) chain_swap<R, X>(v, em); break; \
   case DK_SWAPC + i: if (on) chain_swapc<R, X>(v, em & 0xffffu, em >> 16, op.c); break;
-    switch (h.kind & ~uint32_t(DK_COND)) {
+    switch (skip ? 0u : h.kind & ~uint32_t(DK_COND)) {
       NCSIM_D1(0)
       NCSIM_D1(1)
       NCSIM_D1(2)
@@ -561,9 +570,15 @@ __device__ __forceinline__ void tile_chain(uint32_t tile, uint32_t o, uint32_t g
             if ((em >> b) & 1) turn_in_place(v[b], sx, sy);
         }
         break;
-      case DK_SIGN:
-        if (on) pend ^= em;
+      case DK_SIGNS: {
+        const SignItem* const it = signs + h.gml;
+#pragma unroll 2
+        for (uint32_t i = 0; i < em; ++i) {
+          const SignItem x = it[i];
+          if ((gb & x.fix) == x.fix && (base & x.gfix) == x.gfix) pend ^= x.em;
+        }
         break;
+      }
       case DK_FLUSH: chain_flush<R>(v, pend); break;
       case DK_RZ_OUT: chain_phase<R, -1>(v, op.c[on ? 1 : 0]); break;
       case DK_TABLE: {
@@ -619,7 +634,8 @@ __global__ void __launch_bounds__(3 * PASS_THREADS) k_plain_pass(const __grid_co
   const PassGeom& g = P.g;
   const uint32_t tsz = 1u << g.T;
   OpArgs<R>* const args = reinterpret_cast<OpArgs<R>*>(shared_tile<R>() + 2 * tsz);
-  uint16_t* const cubes = reinterpret_cast<uint16_t*>(args + P.nops);  // chain c, thread t: its cube at c * blockDim.x + t
+  SignItem* const signs = reinterpret_cast<SignItem*>(args + P.nops);
+  uint16_t* const cubes = reinterpret_cast<uint16_t*>(signs + P.nsigns);  // chain c, thread t: its cube at c * blockDim.x + t
   __shared__ uint64_t dround[CUBE];
   // element round r of a thread: elements threadIdx.x + r * blockDim.x
   const uint32_t nr = (tsz + blockDim.x - 1) / blockDim.x;
@@ -629,6 +645,7 @@ __global__ void __launch_bounds__(3 * PASS_THREADS) k_plain_pass(const __grid_co
     const uint4* src = reinterpret_cast<const uint4*>(P.args);
     uint4* dst = reinterpret_cast<uint4*>(args);
     for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+    for (uint32_t i = threadIdx.x; i < P.nsigns; i += blockDim.x) signs[i] = P.sign[i];
   }
   for (uint32_t o = 0; o < P.nops; ++o)
     if (P.head[o].kind == DK_CHAIN) {
@@ -675,7 +692,7 @@ __global__ void __launch_bounds__(3 * PASS_THREADS) k_plain_pass(const __grid_co
     for (uint32_t o = 0; o < P.nops; ++o) {
       const OpHead& h = P.head[o];
       if (h.kind == DK_CHAIN) {
-        tile_chain<R>(buf, o, cubes[h.gvl * blockDim.x + threadIdx.x], args, P, base);
+        tile_chain<R>(buf, o, cubes[h.gvl * blockDim.x + threadIdx.x], args, signs, P, base);
         o += h.em;
       } else {  // DK_TILE_SWAP
         if ((base & P.cond[o].gfix) != P.cond[o].gval) continue;
@@ -909,6 +926,7 @@ struct PlainPlan {
     size_t gate = 0;              // direct: index into `gates`
     Window win;
     std::vector<DevOp> ops;
+    std::vector<SignItem> signs;
   };
   int precision = NCSIM_C128;
   std::vector<const LoweredOp*> gates;
@@ -1045,7 +1063,7 @@ void thread_bits(int T, uint32_t cmask, int SB, uint8_t* at) {
 
 // Groups a pass's ops into chains: maximal runs of consecutive ops whose coupled bits fit in
 // one cube of CUBE_BITS tile bits, each op encoded against its cube.
-std::vector<DevOp> chainify(const std::vector<TileOp>& ops, int T, PlainPlan& P) {
+std::vector<DevOp> chainify(const std::vector<TileOp>& ops, int T, PlainPlan& P, std::vector<SignItem>& signs) {
   std::vector<DevOp> out;
   const auto cst = [&](uint32_t i) { return make_double2(P.cpool[2 * size_t(i)], P.cpool[2 * size_t(i) + 1]); };
   uint32_t chains = 0;
@@ -1148,8 +1166,20 @@ std::vector<DevOp> chainify(const std::vector<TileOp>& ops, int T, PlainPlan& P)
             if (d.h.em == elements(1u << cpos[q], 1u << cpos[q])) half = q;
           const bool all = d.h.em == (1u << CUBE) - 1;
           if (c.x == -1.0 && c.y == 0.0) {
-            d.h.kind = DK_SIGN;
+            // signs that follow one another are one op
             pending = true;
+            if (out.back().h.kind == DK_SIGNS) {
+              ++out.back().h.em;
+              d.h.kind = DK_CHAIN;  // nothing more to add
+            } else {
+              d.h.kind = DK_SIGNS;
+              d.h.gml = uint32_t(signs.size());
+            }
+            signs.push_back({(op.lfix & ~C), d.h.em, op.gfix});
+            if (d.h.kind == DK_CHAIN) continue;
+            d.h.em = 1;
+            d.h.gvl = 0;
+            d.g.gfix = d.g.gval = 0;
           } else if (c.x == 0.0 && (c.y == 1.0 || c.y == -1.0)) {
             d.h.kind = half >= 0 ? DK_TURN + uint32_t(half) : all ? DK_TURN_ALL : DK_TURN_MASK;
             d.x.a[0] = c.y > 0 ? 0x80000000u : 0u;  // i u = (-u.y, u.x)
@@ -1271,7 +1301,7 @@ std::shared_ptr<PlainPlan> plan_plain_passes(uint32_t n, int precision, const st
       it.win = make_window(n, T, moving);
       std::vector<TileOp> ops;
       for (size_t i : cur) ops.push_back(encode(forms[i], it.win, *P));
-      it.ops = chainify(ops, it.win.g.T, *P);
+      it.ops = chainify(ops, it.win.g.T, *P, it.signs);
       if (it.ops.size() > size_t(MAX_PASS_OPS)) throw Error(NCSIM_ERR_INVALID, "tiled pass: too many ops");
       P->passes += 1;
       P->pass_gates += cur.size();
@@ -1311,6 +1341,8 @@ void launch_pass(ncsim_state* s, const PlainPlan& P, const PlainPlan::Item& it) 
   pp.ntiles = s->len >> it.win.g.T;
   pp.nops = uint32_t(it.ops.size());
   pp.nchains = 0;
+  pp.nsigns = uint32_t(it.signs.size());
+  std::copy(it.signs.begin(), it.signs.end(), pp.sign);
   for (size_t i = 0; i < it.ops.size(); ++i) {
     pp.head[i] = it.ops[i].h;
     pp.cond[i] = it.ops[i].g;
@@ -1323,7 +1355,7 @@ void launch_pass(ncsim_state* s, const PlainPlan& P, const PlainPlan::Item& it) 
   pp.cpool = reinterpret_cast<const V<R>*>(P.d_cpool);
   const int T = it.win.g.T;
   const unsigned threads = std::max(32u, 1u << (T - CUBE_BITS));
-  const size_t smem = 2 * (size_t(1) << T) * sizeof(V<R>) + it.ops.size() * sizeof(OpArgs<R>) +
+  const size_t smem = 2 * (size_t(1) << T) * sizeof(V<R>) + it.ops.size() * sizeof(OpArgs<R>) + it.signs.size() * sizeof(SignItem) +
                       size_t(pp.nchains) * threads * sizeof(uint16_t);
   {
     // the kernel's shared-memory limit, set once per device and precision (host threads may race here)
@@ -1334,7 +1366,7 @@ void launch_pass(ncsim_state* s, const PlainPlan& P, const PlainPlan::Item& it) 
     if (dev < 0 || dev >= 64 || !done[dev][sizeof(R) == 8]) {
       NCSIM_CUDA(cudaFuncSetAttribute(
           k_plain_pass<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-          int(2 * (size_t(1) << MAX_TILE_BITS) * sizeof(V<R>) + MAX_PASS_OPS * sizeof(OpArgs<R>) +
+          int(2 * (size_t(1) << MAX_TILE_BITS) * sizeof(V<R>) + MAX_PASS_OPS * (sizeof(OpArgs<R>) + sizeof(SignItem)) +
               MAX_PASS_CHAINS * (1 << (MAX_TILE_BITS - CUBE_BITS)) * sizeof(uint16_t))));
       if (dev >= 0 && dev < 64) done[dev][sizeof(R) == 8] = true;
     }
