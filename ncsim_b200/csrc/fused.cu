@@ -3,29 +3,42 @@
 // A persistent CTA per SM streams tiles of 2^12 complex64 amplitudes (32 KB)
 // through shared memory: two producer warps copy 16-byte chunks with cp.async
 // (completion on the tile's mbarrier through cp.async.mbarrier.arrive) into
-// five rotating tile buffers.  The CTA takes its tiles in sets of four, and
+// five rotating tile buffers, and a third works out what the tile's index bits
+// outside the window decide (which diagonal terms apply, the factor of those
+// that act on the whole tile).  The CTA takes its tiles in sets of four, and
 // four warpgroups run the pass's program, one on each tile of a set, so that a
 // group splits amplitudes while the others' MMAs and read-backs run; each group
 // writes its finished tile back itself (16-byte stores), so the stores overlap
 // the other groups' work and the producers only load.  The unitaries' B
 // operands (16 KB bf16 images each) stream from L2 into three rotating slots
-// (a third producer warp); each group's tcgen05.commit (or release) frees a
+// (a fourth producer warp); each group's tcgen05.commit (or release) frees a
 // slot.  Per group and tile:
 //   unitary op: the tile as 32 rows (the unitary's 5 qubits) x 128 columns;
 //     each thread owns a column, splits its 32 amplitudes into bf16 hi/lo
 //     and writes them into its own TMEM lane (A = X^T, 128 x 64, K-major,
-//     tcgen05.st); one thread issues 12 tcgen05.mma with A in TMEM (M=128,
-//     N=64, K=16, bf16 in, f32 accumulate in the group's 64 TMEM columns):
+//     tcgen05.st); one lane of the group's first warp issues 12 tcgen05.mma
+//     with A in TMEM (M=128, N=64, K=16, bf16 in, f32 accumulate in the
+//     group's 64 TMEM columns):
 //       D = Xhi.Rhi + Xlo.Rhi + Xhi.Rlo
-//     with R the real form [[Ur, -Ui], [Ui, Ur]] of the fused unitary (bf16
-//     hi/lo images made on the host, output columns ordered so that each
-//     row's real and imaginary parts are adjacent); each thread reads its D
-//     row back (tcgen05.ld) and writes the 32 new amplitudes into the tile;
+//     with R the real form of the fused unitary (bf16 hi/lo images made on the
+//     host, output columns ordered so that each row's real and imaginary
+//     parts are adjacent); each thread reads its D row back (tcgen05.ld) and
+//     writes the 32 new amplitudes into the tile;
 //   diagonal op: reduced, where it can be, to a phase per column and a sign
 //     mask over the rows of a neighbouring unitary and applied in that
 //     unitary's split or read-back; otherwise the tile index splits into two
 //     6-bit halves, the active terms fold into a 64-entry phase table per half
 //     and a parity table for cross-half signs, and one sweep applies them.
+// What bounds it (n = 28, 4.4 unitaries a pass): the CUDA cores' work around the
+// MMAs, issue 57% busy, the shared-memory pipe 63%, the tensor pipe 26%, HBM 23%
+// (41% of the time the pass's read and write take).  What the layout of that work
+// measured, n = 28, 5 passes (10.1 ms before): the MMAs issued under elect.sync
+// with warp-uniform operands (12 in 380 cycles, the pipe's own rate; 880 from a
+// thread picked by its index), the tile's facts on a warp of their own, addresses by
+// one XOR, residuals by sub.f32.bf16, signs by two masks a row: 8.0 ms; column bits
+// ordered for free banks and split and read-back loops without conditional updates: 7.65 ms.
+// Tried and slower: one warp issuing every group's MMAs (8.5), two accumulator
+// reads in flight (spills: 9.9), 16-byte moves where row bit 0 is tile bit 0 (8.2).
 // Every wait on an mbarrier is bounded in time: on timeout the CTA records an
 // error code and every role stops at its next uniform decision point, waits
 // for its own copies and frees its TMEM.
@@ -35,6 +48,7 @@
 #include "fused_plan.hpp"
 
 #include <algorithm>
+#include <cstring>
 #include <memory>
 
 namespace ncsim {
@@ -45,25 +59,29 @@ namespace {
 constexpr int GROUP_THREADS = 128;                       // one warpgroup runs the program on one tile
 constexpr int GROUPS = 4;                                // four tiles in flight per CTA
 constexpr int COMPUTE_THREADS = GROUPS * GROUP_THREADS;  // warps 0-15
-constexpr int WARP_TILES = COMPUTE_THREADS / 32;         // warps 16-17: tile loads and stores
+constexpr int WARP_TILES = COMPUTE_THREADS / 32;         // warps 16-17: tile loads
 constexpr int TILE_THREADS = 64;
-constexpr int WARP_OPS = WARP_TILES + 2;                 // warp 18: B operand images
-constexpr int THREADS = COMPUTE_THREADS + TILE_THREADS + 32;
+constexpr int WARP_OPS = WARP_TILES + 2;                 // warp 18: B operand images and MMAs
+constexpr int WARP_FACTS = WARP_OPS + 1;                 // warp 19: what each tile's index bits decide
+constexpr int THREADS = COMPUTE_THREADS + TILE_THREADS + 64;
 constexpr int TILE = 1 << TILE_BITS;
 constexpr uint32_t TILE_BYTES = uint32_t(TILE) * 8u;
 constexpr int OPERAND_BYTES = 16384;  // B: bf16 hi (8 KB) + lo (8 KB)
 constexpr int NTILEBUF = GROUPS + 1;  // tile buffers rotating over the CTA's tiles (one loading ahead)
 constexpr int NOPSLOT = 3;            // B operand slots rotating over the unitary uses
-constexpr int SM_B = 0;
-constexpr int SM_TILE0 = SM_B + NOPSLOT * OPERAND_BYTES;
-constexpr int SM_TOTAL = SM_TILE0 + NTILEBUF * int(TILE_BYTES);
-constexpr int SM_DYNAMIC = SM_TOTAL + 1008;  // the dynamic base is 16-byte aligned: slack to reach 1024
+// Shared memory, from the tiles' base on: the tile buffers sit at multiples of their own size, so
+// a tile element's address is one XOR (base ^ column ^ row); one operand slot lies below them, the
+// others above.  The small tables (struct Tables) fill what is left at the bottom.
+constexpr uint32_t SM_SLOTS = NTILEBUF * TILE_BYTES;
+constexpr uint32_t SM_TPHASE = SM_SLOTS + (NOPSLOT - 1) * uint32_t(OPERAND_BYTES);
+constexpr int MAX_CHUNKS = 48;  // column-term chunks per pass
+constexpr uint32_t SM_END = SM_TPHASE + NTILEBUF * MAX_CHUNKS * uint32_t(sizeof(float2));
+constexpr uint32_t SM_DYNAMIC = TILE_BYTES + SM_END;  // the tiles start within TILE_BYTES of the dynamic base
 // per group 128 columns: the accumulator D (64), the A operand's bf16 hi (32) and lo (32)
 constexpr uint32_t TMEM_COLS = 512;  // 128 per group, rounded up to a power of two
 constexpr long long WAIT_CYCLES = 4000000000ll;  // about 2 s at 1.9 GHz
 constexpr int HALF = TILE_BITS / 2;              // 6-bit halves of the tile index
 constexpr int COL_BITS = TILE_BITS - GROUP_QUBITS;  // a unitary's column index: the tile bits outside its qubits
-constexpr int MAX_CHUNKS = 48;                      // column-term chunks per pass
 // Tile layout in shared memory: element e sits at e ^ L(e), where the linear map L folds
 // tile bits 4..11 into element bits 1..3 (bit j contributes w[j - 4] below).  A unitary's
 // thread owns a column whose 32 lanes step through its lowest non-gate bits; without
@@ -84,7 +102,7 @@ __host__ __device__ inline uint32_t swz_fold(uint32_t e) {
 
 enum TermClass : uint8_t { T_LOW = 0, T_HIGH = 1, T_CROSS_SIGN = 2, T_GENERIC = 3 };
 
-struct OpDesc {
+struct alignas(16) OpDesc {
   uint8_t kind;  // 0 unitary, 1 terms, 2 terms applied by the next unitary's split, 3 by the previous one's read-back
   uint8_t u;     // unitary index (operand slot)
   // terms [t0, t1) sorted by class: low half [t0,tl), high half [tl,th),
@@ -98,7 +116,6 @@ struct TermDesc {
   uint64_t cmask;  // bits outside the window (constant over a tile)
   uint32_t tmask;  // tile-local bits (for a split-applied term: the unitary's non-gate bits)
   float cr, ci;
-  uint32_t rowpat;  // split-applied sign term: the rows (gate index) whose sign flips; 0: a phase on the column
 };
 
 // Up to 32 terms of a diagonal op applied by a unitary's split or read-back,
@@ -106,29 +123,56 @@ struct TermDesc {
 // on a column when its bits outside the tile are set in the tile's base (a
 // per-tile ballot) and its column bits are set in the column index; active
 // terms then flip row signs (row[j]: rows with gate bit j set), negate the
-// column (neg) or multiply it by their phase (gen).
-struct ColChunk {
+// column (neg) or multiply it by their phase (gen; tgen: a phase on every
+// column, folded into one factor per tile; only those that open the op's product,
+// so that the factors multiply in the terms' order whichever way).
+struct alignas(16) ColChunk {
   uint32_t need[COL_BITS];     // terms whose condition includes column bit j
+  uint32_t gen;                // other phases on the whole column
   uint32_t row[GROUP_QUBITS];  // sign terms on the rows with gate bit j set
   uint32_t neg;                // -1 on the whole column
-  uint32_t gen;                // other phases on the whole column
+  uint32_t tgen;               // phases with no column bit, before any in gen: the same on every column
   uint16_t t0;
   uint16_t cnt;
 };
 
-struct PassParams {
-  float2* amp;
-  const uint4* rops;  // nu x 16 KB operand images
-  int* err;
-  uint64_t ntiles;
-  int wl;                      // window bits 0..wl-1 are index bits 0..wl-1
-  uint8_t win[TILE_BITS];      // window qubits, ascending (tile-local bit j = win[j])
-  int nops, nu;
-  uint8_t pos[MAX_UNITARIES][GROUP_QUBITS];  // tile-local positions of each unitary's qubits
-  int nchunks;
+// a pass as the host builds it
+struct PassProgram {
+  int nops, nu, nterms, nchunks;
+  uint8_t pos[MAX_UNITARIES][GROUP_QUBITS];  // tile-local positions of each unitary's qubits (rows)
+  uint8_t col[MAX_UNITARIES][COL_BITS];      // and of the other tile bits (columns), see column_order
   OpDesc ops[MAX_OPS];
   TermDesc terms[MAX_TERMS];
   ColChunk chunks[MAX_CHUNKS];
+};
+struct Terms {
+  uint64_t cmask[MAX_TERMS];
+  float2 coef[MAX_TERMS];
+  uint16_t tmask[MAX_TERMS];
+  __device__ __forceinline__ TermDesc get(int k) const { return {cmask[k], tmask[k], coef[k].x, coef[k].y}; }
+};
+// What a pass's CTAs read with runtime indices: made once with the plan and copied to shared memory
+// by one load per thread.  (Built by every CTA from the program in the kernel's parameters, it took
+// 5000 of the 11000 cycles before the first tile, as much as two unitaries.)
+struct alignas(16) PassTables {
+  ColChunk chunks[MAX_CHUNKS];
+  OpDesc ops[MAX_OPS];
+  alignas(16) uint16_t gbit[MAX_UNITARIES][8];  // byte offset in a tile of each gate bit (row bits)
+  uint16_t clo[MAX_UNITARIES][16];              // byte offset of a column: its low four bits' part
+  uint16_t chi[MAX_UNITARIES][8];               // and its high three bits'
+  uint64_t chunk_off[TILE / 2 / TILE_THREADS];  // byte offset in the register of a tile's 16-byte chunk 64 i
+  Terms terms;
+  uint8_t swz[1 << (TILE_BITS - 4)];            // L(e) by e >> 4
+  uint8_t win[16];                              // tile bit j is index bit win[j], ascending
+  uint8_t out[32];                              // bit j of a tile's number is index bit out[j]
+};
+struct PassArgs {
+  float2* amp;
+  const PassTables* tables;
+  const uint4* rops;  // nu x 16 KB operand images
+  int* err;
+  uint32_t ntiles;
+  int nops, nu, nchunks;
 };
 
 // ---- PTX wrappers ----
@@ -156,8 +200,15 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// one lane of a converged warp; code under it with warp-uniform operands issues tcgen05 at full rate
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
 // bounded wait: false when the phase did not complete within WAIT_CYCLES
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+  if (mbar_try(bar, parity)) return true;
   const long long t0 = clock64();
   while (!mbar_try(bar, parity)) {
     if (clock64() - t0 > WAIT_CYCLES) return false;
@@ -177,7 +228,6 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
-constexpr int BAR_TILES = 1 + GROUPS;  // named barriers: 1..GROUPS the groups, then the tile loaders
 // A named barrier that also ORs a flag over its threads: every thread gets the
 // same answer, so a stop decided from it is uniform across the barrier's threads.
 __device__ __forceinline__ bool bar_any(int id, int count, bool v) {
@@ -206,6 +256,8 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
   return d;
 }
 
+constexpr uint32_t NEGATE_A = 1u << 13;  // instruction descriptor: the product with -A
+
 // D (TMEM) += A (TMEM, K-major rows = lanes) x B (shared memory descriptor)
 __device__ __forceinline__ void mma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile(
@@ -230,50 +282,58 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])    \
                : "r"(taddr))
 
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
+// x, y rounded to bf16, x in the low half
+__device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
+  uint32_t w;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(y), "f"(x));
+  return w;
 }
-// the two bf16 of a packed pair as floats (low half = first element)
-__device__ __forceinline__ float lo_half(uint32_t p) { return __uint_as_float(p << 16); }
-__device__ __forceinline__ float hi_half(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
+// bf16(hi - v) for both halves: minus the residual of v = (x, y) rounded to w
+__device__ __forceinline__ uint32_t pack_neg_residual(uint32_t w, float x, float y) {
+  float a, b;
+  asm("{\n\t.reg .b16 p, q;\n\tmov.b32 {p, q}, %2;\n\tsub.f32.bf16 %0, p, %3;\n\tsub.f32.bf16 %1, q, %4;\n\t}"
+      : "=f"(a), "=f"(b)
+      : "r"(w), "f"(x), "f"(y));
+  return pack_bf16(a, b);
+}
+// an amplitude at a shared-memory address (program order among these and the barriers: volatile)
+__device__ __forceinline__ void lds_amp(uint32_t at, float& x, float& y) {
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(at));
+}
+__device__ __forceinline__ void sts_amp(uint32_t at, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(x), "r"(y));
+}
 
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// index of tile-local element e of a tile whose base index is `base`
-__device__ __forceinline__ uint64_t global_index(uint64_t base, uint32_t e, const PassParams& P) {
-  uint64_t g = base | (e & ((1u << P.wl) - 1));
-  for (int j = P.wl; j < TILE_BITS; ++j) g |= uint64_t((e >> j) & 1u) << P.win[j];
-  return g;
-}
-// the tile's base: the tile number deposited into the bits outside the window
-__device__ __forceinline__ uint64_t tile_base(uint64_t t, const PassParams& P) {
-  uint64_t v = t;
-  for (int j = 0; j < TILE_BITS; ++j) {
-    const int b = P.win[j];
-    v = ((v >> b) << (b + 1)) | (v & ((uint64_t(1) << b) - 1));
-  }
-  return v;
-}
-
+struct Tables : PassTables {
+  uint64_t bars[2 * NTILEBUF + 2 * NOPSLOT + 2 * GROUPS];  // tile full, tile done, operand full, operand empty, split, mma
+  float2 tab_lo[GROUPS][1 << HALF], tab_hi[GROUPS][1 << HALF];
+  uint8_t tab_cross[GROUPS][1 << HALF];
+  uint32_t act[NTILEBUF][MAX_CHUNKS];          // per tile: the chunks' terms active on it
+  uint64_t base[NTILEBUF];                     // and its first index
+  uint32_t tmem_base;
+  volatile int abort;
+};
+static_assert(sizeof(Tables) + 1024 + uint32_t(OPERAND_BYTES) <= TILE_BYTES, "the small tables fit below the first operand slot");
 // The tile's phase tables of a terms op, built by one group's 128 threads: the
 // low-half phase products and cross-half sign parities (threads 0-63) and the
 // high-half phase products (64-127).
-__device__ __forceinline__ void build_tables(const OpDesc& op, uint64_t base, int tg, const TermDesc* terms,
+__device__ __forceinline__ void build_tables(const OpDesc& op, uint64_t base, int tg, const Terms& terms,
                                              float2* tab_lo, float2* tab_hi, uint8_t* tab_cross) {
   if (tg < 64) {
     const uint32_t x = uint32_t(tg);
     float2 c = make_float2(1.f, 0.f);
     for (int k = op.t0; k < op.tl; ++k) {
-      const TermDesc tm = terms[k];
+      const TermDesc tm = terms.get(k);
       if ((base & tm.cmask) == tm.cmask && (x & tm.tmask) == tm.tmask) c = cmulf(c, make_float2(tm.cr, tm.ci));
     }
     tab_lo[x] = c;
     uint32_t v = 0;
     for (int k = op.th; k < op.tc; ++k) {
-      const TermDesc tm = terms[k];
+      const TermDesc tm = terms.get(k);
       if ((base & tm.cmask) != tm.cmask) continue;
       if (x & (tm.tmask >> HALF)) v ^= tm.tmask & ((1u << HALF) - 1);
     }
@@ -282,7 +342,7 @@ __device__ __forceinline__ void build_tables(const OpDesc& op, uint64_t base, in
     const uint32_t x = uint32_t(tg - 64);
     float2 c = make_float2(1.f, 0.f);
     for (int k = op.tl; k < op.th; ++k) {
-      const TermDesc tm = terms[k];
+      const TermDesc tm = terms.get(k);
       const uint32_t hm = tm.tmask >> HALF;
       if ((base & tm.cmask) == tm.cmask && (x & hm) == hm) c = cmulf(c, make_float2(tm.cr, tm.ci));
     }
@@ -291,228 +351,274 @@ __device__ __forceinline__ void build_tables(const OpDesc& op, uint64_t base, in
 }
 
 // the phase of tile element e under a terms op (its tables built)
-__device__ __forceinline__ float2 term_phase(uint32_t e, const OpDesc& op, uint64_t base, const TermDesc* terms,
+__device__ __forceinline__ float2 term_phase(uint32_t e, const OpDesc& op, uint64_t base, const Terms& terms,
                                              const float2* tab_lo, const float2* tab_hi, const uint8_t* tab_cross) {
   const uint32_t lo = e & ((1u << HALF) - 1), hi = e >> HALF;
   float2 c = cmulf(tab_lo[lo], tab_hi[hi]);
   if (__popc(lo & tab_cross[hi]) & 1) c = make_float2(-c.x, -c.y);
   for (int k = op.tc; k < op.t1; ++k) {
-    const TermDesc tm = terms[k];
+    const TermDesc tm = terms.get(k);
     if ((base & tm.cmask) == tm.cmask && (e & tm.tmask) == tm.tmask) c = cmulf(c, make_float2(tm.cr, tm.ci));
   }
   return c;
 }
 
 // The chunks [c0, c1) of a diagonal op applied by a unitary's split or read-back,
-// for column tg of that unitary (act: the chunks' terms active on this tile):
-// a sign mask over the 32 rows and a phase for the whole column.
-__device__ __forceinline__ void column_chunks(const ColChunk* chunks, const uint32_t* act, int c0, int c1, uint32_t tg,
-                                              const TermDesc* terms, uint32_t& smask, float2& cth, bool& scal) {
-  const uint32_t rowpat[GROUP_QUBITS] = {0xAAAAAAAAu, 0xCCCCCCCCu, 0xF0F0F0F0u, 0xFF00FF00u, 0xFFFF0000u};
+// for column tg of that unitary (act: the chunks' terms active on this tile, without the
+// tgen ones, whose product is tph).  par: bit j, the rows with gate bit j set change sign;
+// bit 5, every row does.  cth: a phase for the whole column (scal: there is one).
+__device__ __forceinline__ void column_chunks(const ColChunk* chunks, const uint32_t* act, const float2* tph, int c0, int c1,
+                                              uint32_t tg, const float2* coef, uint32_t& par, float2& cth, bool& scal) {
   for (int c = c0; c < c1; ++c) {
-    const ColChunk& ch = chunks[c];
+    ColChunk ch;
+    {
+      const uint4* const from = reinterpret_cast<const uint4*>(chunks + c);
+      uint4* const to = reinterpret_cast<uint4*>(&ch);
+#pragma unroll
+      for (int i = 0; i < int(sizeof(ColChunk) / 16); ++i) to[i] = from[i];
+    }
     uint32_t a = act[c];
 #pragma unroll
     for (int j = 0; j < COL_BITS; ++j) a &= ((tg >> j) & 1u) ? ~0u : ~ch.need[j];
 #pragma unroll
-    for (int j = 0; j < GROUP_QUBITS; ++j) smask ^= rowpat[j] & (0u - (uint32_t(__popc(a & ch.row[j])) & 1u));
-    if (__popc(a & ch.neg) & 1) {
-      cth = make_float2(-cth.x, -cth.y);
+    for (int j = 0; j < GROUP_QUBITS; ++j) par ^= (uint32_t(__popc(a & ch.row[j])) & 1u) << j;
+    par ^= (uint32_t(__popc(a & ch.neg)) & 1u) << GROUP_QUBITS;
+    if (ch.tgen) {
+      cth = cmulf(cth, tph[c]);
       scal = true;
     }
     for (uint32_t gb = a & ch.gen; gb; gb &= gb - 1) {
-      const TermDesc& td = terms[ch.t0 + (__ffs(gb) - 1)];
-      cth = cmulf(cth, make_float2(td.cr, td.ci));
+      cth = cmulf(cth, coef[ch.t0 + (__ffs(gb) - 1)]);
       scal = true;
     }
   }
+}
+// The sign words of 32 rows: row 8 q + i flips by m8[i] ^ m4[q].
+__device__ __forceinline__ void sign_words(uint32_t par, uint32_t (&m8)[8], uint32_t (&m4)[4]) {
+  uint32_t m[GROUP_QUBITS + 1];
+#pragma unroll
+  for (int j = 0; j <= GROUP_QUBITS; ++j) m[j] = (0u - ((par >> j) & 1u)) & 0x80000000u;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) m8[i] = ((i & 1) ? m[0] : 0u) ^ ((i & 2) ? m[1] : 0u) ^ ((i & 4) ? m[2] : 0u);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) m4[q] = ((q & 1) ? m[3] : 0u) ^ ((q & 2) ? m[4] : 0u) ^ m[5];
+}
+// The same for packed pairs of bf16: rows 8 q + 2 i (low half) and the next flip by mp[i] ^ m4[q].
+__device__ __forceinline__ void sign_pairs(uint32_t par, uint32_t (&mp)[4], uint32_t (&m4)[4]) {
+  uint32_t m[GROUP_QUBITS + 1];
+#pragma unroll
+  for (int j = 0; j <= GROUP_QUBITS; ++j) m[j] = (0u - ((par >> j) & 1u)) & (j ? 0x80008000u : 0x80000000u);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) mp[i] = m[0] ^ ((i & 1) ? m[1] : 0u) ^ ((i & 2) ? m[2] : 0u);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) m4[q] = ((q & 1) ? m[3] : 0u) ^ ((q & 2) ? m[4] : 0u) ^ m[5];
 }
 
 __device__ __forceinline__ void bar_group(int g) {
   asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(GROUP_THREADS) : "memory");
 }
 
-__global__ void __launch_bounds__(THREADS, 1) k_fused_pass(const __grid_constant__ PassParams P) {
-  extern __shared__ uint8_t smem_raw[];
-  // 1024-byte aligned (the swizzled operand images); an offset into the shared array keeps the
-  // pointers in the shared address space (32-bit addressing for every tile access)
-  uint8_t* smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
-  // mbarriers: tile full[3], tile done[3], operand full[3], operand empty[3], mma[2]
-  __shared__ __align__(8) uint64_t bars[2 * NTILEBUF + 2 * NOPSLOT + GROUPS];
-  __shared__ uint32_t tmem_base_sh;
-  __shared__ volatile int abort_sh;
-  __shared__ uint16_t nbit[MAX_UNITARIES][COL_BITS];       // stored offset of each non-gate bit (column bits)
-  __shared__ uint16_t gbit[MAX_UNITARIES][GROUP_QUBITS];   // and of each gate bit (row bits)
-  __shared__ uint8_t swz[1 << (TILE_BITS - 4)];             // L(e) by e >> 4
-  __shared__ float2 tab_lo[GROUPS][1 << HALF], tab_hi[GROUPS][1 << HALF];
-  __shared__ uint8_t tab_cross[GROUPS][1 << HALF];
-  __shared__ uint64_t run_off[TILE >> LOW_BITS];  // index bits of run r of a tile (the window bits above wl)
-  __shared__ TermDesc s_terms[MAX_TERMS];         // the pass's program, read with runtime indices
-  __shared__ OpDesc s_ops[MAX_OPS];
-  __shared__ ColChunk s_chunks[MAX_CHUNKS];
-  __shared__ uint32_t act_sh[GROUPS][MAX_CHUNKS];  // per tile: the chunks' terms active on it
+// NG: the warpgroups that work, and so the tiles in a set (a run-time count made the full kernel 7% slower)
+template <uint32_t NG>
+__global__ void __launch_bounds__(THREADS, 1) k_fused_pass(const __grid_constant__ PassArgs P) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  Tables& S = *reinterpret_cast<Tables*>(smem_raw);
+  const uint32_t sm0 = smem_u32(smem_raw);
+  const uint32_t tiles0 = (sm0 + uint32_t(sizeof(Tables)) + uint32_t(OPERAND_BYTES) + TILE_BYTES - 1) & ~(TILE_BYTES - 1);
+  if (tiles0 + SM_END > sm0 + SM_DYNAMIC) {  // every thread alike, before anything is held
+    if (threadIdx.x == 0) atomicCAS(P.err, 0, 5);
+    return;
+  }
+  // operand slot 0 ends where the tiles begin, the others follow the tiles
+  auto slot_addr = [&](uint32_t s) { return s ? tiles0 + SM_SLOTS + (s - 1) * OPERAND_BYTES : tiles0 - OPERAND_BYTES; };
+  float2* const tphase_sh = reinterpret_cast<float2*>(smem_raw + (tiles0 - sm0) + SM_TPHASE);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  auto bar_tfull = [&](int b) { return smem_u32(&bars[b]); };
-  auto bar_tdone = [&](int b) { return smem_u32(&bars[NTILEBUF + b]); };
-  auto bar_ofull = [&](int s) { return smem_u32(&bars[2 * NTILEBUF + s]); };
-  auto bar_oempty = [&](int s) { return smem_u32(&bars[2 * NTILEBUF + NOPSLOT + s]); };
-  auto bar_mma = [&](int g) { return smem_u32(&bars[2 * NTILEBUF + 2 * NOPSLOT + g]); };
+  auto bar_tfull = [&](uint32_t b) { return smem_u32(&S.bars[b]); };
+  auto bar_tdone = [&](uint32_t b) { return smem_u32(&S.bars[NTILEBUF + b]); };
+  auto bar_ofull = [&](uint32_t s) { return smem_u32(&S.bars[2 * NTILEBUF + s]); };
+  auto bar_oempty = [&](uint32_t s) { return smem_u32(&S.bars[2 * NTILEBUF + NOPSLOT + s]); };
+  auto bar_split = [&](int g) { return smem_u32(&S.bars[2 * NTILEBUF + 2 * NOPSLOT + g]); };
+  auto bar_mma = [&](int g) { return smem_u32(&S.bars[2 * NTILEBUF + 2 * NOPSLOT + GROUPS + g]); };
   auto fail = [&](int code) {
-    abort_sh = 1;
+    S.abort = 1;
     atomicCAS(P.err, 0, code);
   };
 
   if (tid == 0) {
     for (int i = 0; i < NTILEBUF; ++i) {
-      mbar_init(bar_tfull(i), TILE_THREADS);  // one cp.async arrival per tile thread
-      mbar_init(bar_tdone(i), GROUP_THREADS);
+      mbar_init(bar_tfull(i), TILE_THREADS + 1);  // one cp.async arrival per tile thread, one for the tile's facts
+      mbar_init(bar_tdone(i), GROUP_THREADS / 32);
     }
     for (int i = 0; i < NOPSLOT; ++i) {
       mbar_init(bar_ofull(i), 1);
-      mbar_init(bar_oempty(i), GROUPS);  // one commit (or release) per group
+      mbar_init(bar_oempty(i), NG);  // one commit (or release) per group
     }
-    for (int g = 0; g < GROUPS; ++g) mbar_init(bar_mma(g), 1);
-    abort_sh = 0;
+    for (int g = 0; g < GROUPS; ++g) {
+      mbar_init(bar_split(g), GROUP_THREADS / 32);
+      mbar_init(bar_mma(g), 1);
+    }
+    S.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)),
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&S.tmem_base)),
                  "r"(TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  for (uint32_t r = uint32_t(tid); r < (uint32_t(TILE) >> P.wl); r += THREADS) run_off[r] = global_index(0, r << P.wl, P);
-  for (uint32_t h = uint32_t(tid); h < (1u << (TILE_BITS - 4)); h += THREADS) swz[h] = uint8_t(swz_fold(h << 4));
-  for (int i = tid; i < P.nops; i += THREADS) s_ops[i] = P.ops[i];
-  for (int i = tid; i < P.nchunks; i += THREADS) s_chunks[i] = P.chunks[i];
-  {
-    int nterms = 0;
-    for (int i = 0; i < P.nops; ++i) nterms = max(nterms, int(P.ops[i].t1));
-    for (int i = tid; i < nterms; i += THREADS) s_terms[i] = P.terms[i];
-  }
-  for (int u = tid; u < P.nu; u += THREADS) {  // the non-gate tile bits of each unitary
-    uint32_t gm = 0;
-    for (int j = 0; j < GROUP_QUBITS; ++j) gm |= 1u << P.pos[u][j];
-    int m = 0;
-    for (int b = 0; b < TILE_BITS; ++b)
-      if (!((gm >> b) & 1)) nbit[u][m++] = uint16_t((1u << b) ^ swz_fold(1u << b));
-    for (int j = 0; j < GROUP_QUBITS; ++j) gbit[u][j] = uint16_t((1u << P.pos[u][j]) ^ swz_fold(1u << P.pos[u][j]));
-  }
+  for (uint32_t i = uint32_t(tid); i < uint32_t(sizeof(PassTables) / 16); i += THREADS)
+    reinterpret_cast<uint4*>(smem_raw)[i] = __ldg(reinterpret_cast<const uint4*>(P.tables) + i);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_sh;
-  // tiles go in groups of GROUPS, one per warpgroup: this CTA's it-th tile is tile_of(it),
-  // in buffer it % NTILEBUF; only the register's last group of tiles can be short, and it
-  // is the last one of the CTA that takes it
-  const uint64_t nsets = (P.ntiles + GROUPS - 1) / GROUPS;
-  const uint64_t my_sets = nsets > blockIdx.x ? (nsets - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const uint64_t my_tiles = uint64_t(GROUPS) * my_sets;
-  auto tile_of = [&](uint64_t it) {
-    return uint64_t(GROUPS) * (uint64_t(blockIdx.x) + (it / GROUPS) * gridDim.x) + (it % GROUPS);
-  };
-  auto have = [&](uint64_t it) { return tile_of(it) < P.ntiles; };
-  float2* tiles = reinterpret_cast<float2*>(smem + SM_TILE0);
-  auto at = [&](uint32_t e) { return e ^ uint32_t(swz[e >> 4]); };  // stored position of tile element e
-  const uint32_t cshift = uint32_t(P.wl) - 1u;  // 16-byte chunks of 2 amplitudes per run: 2^(wl-1)
-  auto chunk_addr = [&](uint64_t base, uint32_t c) {
-    return P.amp + (base | run_off[c >> cshift]) + 2u * (c & ((1u << cshift) - 1u));
+  const uint32_t tmem = __shfl_sync(0xffffffffu, S.tmem_base, 0);
+  // tiles go in sets of NG, one per warpgroup: tile j of this CTA's set p is tile_of(p, j) and
+  // the CTA's it-th, in buffer it % NTILEBUF; only the register's last set of tiles can be short,
+  // and it is the last one of the CTA that takes it
+  const uint32_t ntiles = P.ntiles;
+  const uint32_t nsets = (ntiles + NG - 1) / NG;
+  const uint32_t my_sets = nsets > blockIdx.x ? (nsets - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+  auto tile_of = [&](uint32_t p, uint32_t j) { return NG * (blockIdx.x + p * gridDim.x) + j; };
+  float2* tiles = reinterpret_cast<float2*>(smem_raw + (tiles0 - sm0));
+  auto at = [&](uint32_t e) { return e ^ uint32_t(S.swz[e >> 4]); };  // stored position of tile element e
+  // byte offset in the register of a tile's 16-byte chunk c < 128; chunks of disjoint bits add
+  auto chunk_off = [&](uint32_t c) {
+    uint64_t g = 0;
+#pragma unroll
+    for (int j = 0; j < 7; ++j) g |= uint64_t((c >> j) & 1u) << S.win[j + 1];
+    return g * sizeof(float2);
   };
 
-  if (warp == WARP_TILES || warp == WARP_TILES + 1) {
-    // ---------------- tile loads (cp.async): 64 threads, 16-byte chunks ----------------
+  if (warp >= WARP_TILES && warp != WARP_OPS) {
+    // ---------------- tiles in order: their loads (64 threads), their facts (a warp) ----------------
+    const bool facts = warp == WARP_FACTS;
     const int pt = tid - COMPUTE_THREADS;
-    auto load_tile = [&](uint64_t it) {
-      const int b = int(it % NTILEBUF);
-      const uint64_t base = tile_base(tile_of(it), P);
-      const uint32_t dst = smem_u32(tiles + size_t(b) * TILE);
-#pragma unroll 4
-      for (uint32_t c = uint32_t(pt); c < uint32_t(TILE) / 2; c += TILE_THREADS) cp_async16(dst + 8u * at(2u * c), chunk_addr(base, c));
-      cp_async_arrive(bar_tfull(b));
-    };
-    // wait (one thread) until the group has written tile j back; false (for all 64 threads alike) to stop
-    auto wait_done = [&](uint64_t j) -> bool {
-      if (pt == 0 && have(j) && !mbar_wait(bar_tdone(int(j % NTILEBUF)), uint32_t((j / NTILEBUF) & 1))) fail(3);
-      return !bar_any(BAR_TILES, TILE_THREADS, abort_sh);
-    };
-    for (uint64_t it = 0; it < my_tiles; ++it) {
-      if (it >= NTILEBUF && !wait_done(it - NTILEBUF)) break;  // the buffer is free once its tile is written back
-      if (have(it)) load_tile(it);
+    const uint64_t my_off = chunk_off(uint32_t(pt) & (TILE_THREADS - 1));
+    const uint32_t my_at = 8u * at(2u * (uint32_t(pt) & (TILE_THREADS - 1)));  // positions of disjoint bits combine by XOR
+    const uint64_t lane_bit = uint64_t(1) << S.out[lane];  // the index bit that bit `lane` of a tile number stands for
+    uint32_t b = 0, parity = 1;  // buffer it % NTILEBUF, and the parity of its last use
+    for (uint32_t it = 0, p = 0, j = 0; p < my_sets; ++it) {
+      const uint32_t t = tile_of(p, j);
+      if (t >= ntiles) break;  // the CTA's last tiles
+      if (++j == NG) j = 0, ++p;
+      if (it >= NTILEBUF) {    // the buffer is free once its last tile is written back; each warp stops by itself
+        bool ok = true;
+        if (lane == 0) {
+          ok = mbar_wait(bar_tdone(b), parity);
+          if (!ok) fail(3);
+          ok = ok && !S.abort;
+        }
+        if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+      }
+      const bool on = (t >> lane) & 1u;
+      const uint64_t base = uint64_t(__reduce_or_sync(0xffffffffu, on ? uint32_t(lane_bit >> 32) : 0u)) << 32 |
+                            __reduce_or_sync(0xffffffffu, on ? uint32_t(lane_bit) : 0u);
+      if (!facts) {
+        const uint8_t* const src = reinterpret_cast<const uint8_t*>(P.amp) + base * sizeof(float2) + my_off;
+        const uint32_t dst = (tiles0 + b * TILE_BYTES) ^ my_at;
+#pragma unroll 8
+        for (uint32_t i = 0; i < uint32_t(TILE / 2 / TILE_THREADS); ++i) {
+          const uint32_t e = 2u * TILE_THREADS * i;
+          cp_async16(dst ^ (8u * (e ^ swz_fold(e))), src + S.chunk_off[i]);
+        }
+        cp_async_arrive(bar_tfull(b));
+      } else {
+        // which column terms apply on this tile (their bits outside it)
+        for (int c = 0; c < P.nchunks; ++c) {
+          const ColChunk& ch = S.chunks[c];
+          const uint64_t cm = lane < int(ch.cnt) ? S.terms.cmask[ch.t0 + lane] : 0;
+          const bool act = lane < int(ch.cnt) && (base & cm) == cm;
+          const uint32_t m = __ballot_sync(0xffffffffu, act);
+          if (ch.tgen) {  // the same phase on every column: their product, once
+            float2 f = make_float2(1.f, 0.f);
+            for (uint32_t gb = m & ch.tgen; gb; gb &= gb - 1) f = cmulf(f, S.terms.coef[ch.t0 + (__ffs(gb) - 1)]);
+            if (lane == 0) tphase_sh[b * MAX_CHUNKS + c] = f;
+          }
+          if (lane == 0) S.act[b][c] = m & ~ch.tgen;
+        }
+        if (lane == 0) {
+          S.base[b] = base;
+          mbar_arrive(bar_tfull(b));
+        }
+      }
+      if (++b == NTILEBUF) b = 0, parity ^= 1u;
     }
     // copies of this thread still in flight land before the CTA exits
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == WARP_OPS) {
     // ---------------- B operand images: use k = set * nu + u, slot k % NOPSLOT ----------------
-    const uint64_t nk = my_sets * uint64_t(P.nu);
-    uint64_t k = 0;
+    const uint32_t nk = my_sets * uint32_t(P.nu);
+    uint32_t k = 0, sl = 0, parity = 1, u = 0;
     for (; k < nk; ++k) {
-      const int sl = int(k % NOPSLOT);
       if (k >= NOPSLOT) {
         bool go = true;
         if (lane == 0) {
-          go = mbar_wait(bar_oempty(sl), uint32_t(((k - NOPSLOT) / NOPSLOT) & 1));
+          go = mbar_wait(bar_oempty(sl), parity);
           if (!go) fail(4);
-          go = go && !abort_sh;
+          go = go && !S.abort;
         }
         if (!__shfl_sync(0xffffffffu, go, 0)) break;  // lane 0 decides for the warp
       }
       if (lane == 0) {
         mbar_expect_tx(bar_ofull(sl), OPERAND_BYTES);
-        bulk_load(smem_u32(smem + SM_B + sl * OPERAND_BYTES), P.rops + (k % uint64_t(P.nu)) * (OPERAND_BYTES / 16),
-                  OPERAND_BYTES, bar_ofull(sl));
+        bulk_load(slot_addr(sl), P.rops + u * (OPERAND_BYTES / 16), OPERAND_BYTES, bar_ofull(sl));
       }
       __syncwarp();
+      if (++u == uint32_t(P.nu)) u = 0;
+      if (++sl == NOPSLOT) sl = 0, parity ^= 1u;
     }
     if (k < nk)  // an abort: let the loads already issued land
-      for (uint64_t j = k >= NOPSLOT ? k - NOPSLOT : 0; j < k; ++j)
-        if (lane == 0) mbar_wait(bar_ofull(int(j % NOPSLOT)), uint32_t((j / NOPSLOT) & 1));
+      for (uint32_t j = k >= NOPSLOT ? k - NOPSLOT : 0; j < k; ++j)
+        if (lane == 0) mbar_wait(bar_ofull(j % NOPSLOT), (j / NOPSLOT) & 1);
   } else {
     // ---------------- tensor-core program: group g on its tile of each set ----------------
     const int g = warp / 4, tg = tid & (GROUP_THREADS - 1);
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
-    const uint32_t d_tmem = tmem + uint32_t(128 * g);  // columns: D [0,64), A hi [64,96), A lo [96,128)
-    const uint32_t a_tmem = d_tmem + 64u;
     const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
-    const uint32_t taddr = d_tmem + lane_base;          // this warp's lanes of D
-    const uint32_t taddr_a = a_tmem + lane_base;        // and of A
+    const uint32_t taddr = tmem + uint32_t(128 * g) + lane_base;  // this warp's lanes: D [0,64), A hi [64,96), A lo [96,128)
+    const uint32_t taddr_a = taddr + 64u;
+    // the group's first warp issues its MMAs; warp-uniform operands
+    const int gu = __shfl_sync(0xffffffffu, g, 0);
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+    const uint32_t d_tmem = tmem + uint32_t(128 * gu), a_tmem = d_tmem + 64u;
+    uint32_t sl = 0, sl_phase = 0;  // the next use's operand slot
     uint32_t mma_phase = 0;
-    for (uint64_t p = 0; p < my_sets; ++p) {
-      const uint64_t it = uint64_t(GROUPS) * p + uint64_t(g);
-      const bool mine = have(it);
-      const int b = int(it % NTILEBUF);
-      const uint64_t base = mine ? tile_base(tile_of(it), P) : 0;
-      if (mine && tg < 32) {  // which column terms apply on this tile (their bits outside it)
-        for (int c = 0; c < P.nchunks; ++c) {
-          bool on = false;
-          if (tg < int(s_chunks[c].cnt)) {
-            const uint64_t cm = s_terms[s_chunks[c].t0 + tg].cmask;
-            on = (base & cm) == cm;
+    const uint64_t my_off = chunk_off(uint32_t(tg));
+    const uint32_t my_at = 8u * at(2u * uint32_t(tg));
+    uint32_t b = uint32_t(g), parity = 0;  // buffer of this group's tile, and the parity of its use
+    for (uint32_t p = 0; p < my_sets && uint32_t(g) < NG; ++p) {
+      if (tile_of(p, uint32_t(g)) >= ntiles) {  // no tile in the last set: release its operand slots unused
+        if (tg == 0)
+          for (int u = 0; u < P.nu && !S.abort; ++u) {
+            if (!mbar_wait(bar_ofull(sl), sl_phase)) fail(2);
+            mbar_arrive(bar_oempty(sl));
+            if (++sl == NOPSLOT) sl = 0, sl_phase ^= 1u;
           }
-          const uint32_t m = __ballot_sync(0xffffffffu, on);
-          if (tg == 0) act_sh[g][c] = m;
-        }
+        break;
       }
-      if (mine && tg == 0 && !mbar_wait(bar_tfull(b), uint32_t((it / NTILEBUF) & 1))) fail(1);
-      if (bar_any(1 + g, GROUP_THREADS, abort_sh)) break;
+      if (!mbar_wait(bar_tfull(b), parity)) fail(1);
+      const uint64_t base = S.base[b];
       float2* T = tiles + size_t(b) * TILE;
+      const uint32_t* const act = S.act[b];
+      const float2* const tph = tphase_sh + b * MAX_CHUNKS;
+      bool stop = false;
       for (int oi = 0; oi < P.nops; ++oi) {
-        const OpDesc op = s_ops[oi];
-        if (op.kind >= 2) continue;  // applied by a neighbouring unitary's split or read-back
+        const uint4 opw = *reinterpret_cast<const uint4*>(&S.ops[oi]);
+        OpDesc op;
+        *reinterpret_cast<uint4*>(&op) = opw;
         if (op.kind == 1) {
-          if (!mine) continue;
           // ---- diagonal terms: per-tile tables, then one sweep of the tile ----
-          build_tables(op, base, tg, s_terms, tab_lo[g], tab_hi[g], tab_cross[g]);
+          build_tables(op, base, tg, S.terms, S.tab_lo[g], S.tab_hi[g], S.tab_cross[g]);
           bar_group(g);
           {
             // element e = tg + 128 i: its low 6 bits are the thread's, so the low-half
             // phase is one read; the high-half entries are the same across a warp
             const uint32_t lo = uint32_t(tg) & ((1u << HALF) - 1);
-            const float2 L = tab_lo[g][lo];
+            const float2 L = S.tab_lo[g][lo];
             if (op.tc == op.t1) {
               // blocks of 8: every load before any store (the tile and the tables may alias as far
               // as the compiler knows, so a store would hold back the next loads)
-              const float2* __restrict__ th = tab_hi[g];
-              const uint8_t* __restrict__ tx = tab_cross[g];
+              const float2* __restrict__ th = S.tab_hi[g];
+              const uint8_t* __restrict__ tx = S.tab_cross[g];
 #pragma unroll 1
               for (int i0 = 0; i0 < TILE / GROUP_THREADS; i0 += 8) {
                 float2 v[8], h[8];
@@ -536,7 +642,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused_pass(const __grid_constant
 #pragma unroll 4
               for (int i = 0; i < TILE / GROUP_THREADS; ++i) {
                 const uint32_t e = uint32_t(tg + GROUP_THREADS * i);
-                T[at(e)] = cmulf(term_phase(e, op, base, s_terms, tab_lo[g], tab_hi[g], tab_cross[g]), T[at(e)]);
+                T[at(e)] = cmulf(term_phase(e, op, base, S.terms, S.tab_lo[g], S.tab_hi[g], S.tab_cross[g]), T[at(e)]);
               }
             }
           }
@@ -545,140 +651,184 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused_pass(const __grid_constant
         }
         // ---- unitary op: this thread owns column tg (A row / TMEM lane) and its 32 rows ----
         const int u = op.u;
-        const uint64_t k = p * uint64_t(P.nu) + uint64_t(u);
-        const int sl = int(k % NOPSLOT);
-        if (!mine) {
-          // this group has no tile in the set: release the operand slot without using it
-          if (abort_sh) break;
-          if (tg == 0) {
-            if (!mbar_wait(bar_ofull(sl), uint32_t((k / NOPSLOT) & 1))) fail(2);
-            mbar_arrive(bar_oempty(sl));
-          }
-          continue;
-        }
         // stored positions (the layout fold is linear: column and row parts combine by XOR)
-        uint32_t cb = 0;
-#pragma unroll
-        for (int j = 0; j < COL_BITS; ++j) cb ^= ((tg >> j) & 1) ? uint32_t(nbit[u][j]) : 0u;
-        const uint32_t p0 = gbit[u][0], p1 = gbit[u][1], p2 = gbit[u][2], p3 = gbit[u][3], p4 = gbit[u][4];
+        const uint32_t cb = (tiles0 + b * TILE_BYTES) ^ uint32_t(S.clo[u][tg & 15]) ^ uint32_t(S.chi[u][tg >> 4]);
+        const uint4 gb = *reinterpret_cast<const uint4*>(S.gbit[u]);
+        const uint32_t p0 = gb.x & 0xffffu, p1 = gb.x >> 16, p2 = gb.y & 0xffffu, p3 = gb.y >> 16, p4 = gb.z & 0xffffu;
         uint32_t lo8[8];  // rows 0..7 (gate bits 0-2) of this column
 #pragma unroll
         for (int i = 0; i < 8; ++i) lo8[i] = cb ^ ((i & 1) ? p0 : 0u) ^ ((i & 2) ? p1 : 0u) ^ ((i & 4) ? p2 : 0u);
         const uint32_t hi4[4] = {0u, p3, p4, p3 ^ p4};  // rows 8q..8q+7
-        // a preceding diagonal op, reduced to this column: a phase and a sign mask over the 32 rows
-        uint32_t smask = 0;
+        // a preceding diagonal op, reduced to this column: a sign per row and a phase of the column
+        uint32_t par = 0;
         float2 cth = make_float2(1.f, 0.f);
         bool scal = false;
-        column_chunks(s_chunks, act_sh[g], op.pc0, op.pc1, uint32_t(tg), s_terms, smask, cth, scal);
+        column_chunks(S.chunks, act, tph, op.pc0, op.pc1, uint32_t(tg), S.terms.coef, par, cth, scal);
         // warp-uniform decisions (a lane without a phase multiplies by exactly 1, one without
         // signs flips nothing), so the unrolled loops carry no divergent branches
         scal = __any_sync(0xffffffffu, scal);
-        const bool flip = __any_sync(0xffffffffu, smask != 0);
+        const bool flip = __any_sync(0xffffffffu, par != 0);
+        // the previous op's stores are in, and everyone stops alike
+        stop = bar_any(1 + g, GROUP_THREADS, S.abort);
+        if (stop) break;
+        // A row (this lane): K = row (real parts) and 32 + row (imaginary parts), two bf16 per
+        // column, so rows 8q .. 8q+7 are columns 4q .. 4q+3 (re) and 16 + the same (im).  One loop
+        // per kind: in one loop, results kept in place past a branch cost a register copy each.
+        if (scal) {
+          uint32_t mp[4], m4[4];
+          sign_pairs(par, mp, m4);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float2 xx[8];  // rows 8q..8q+7, loaded before any other work
+          for (int q = 0; q < 4; ++q) {
+            float x[8], y[8];  // rows 8q..8q+7, loaded before any other work
 #pragma unroll
-          for (int i = 0; i < 8; ++i) xx[i] = T[lo8[i] ^ hi4[q]];
-          if (scal) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) xx[i] = cmulf(cth, xx[i]);
-          }
-          if (flip) {
+            for (int i = 0; i < 8; ++i) lds_amp(lo8[i] ^ hi4[q], x[i], y[i]);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              const uint32_t sg = (smask << (31 - (8 * q + i))) & 0x80000000u;
-              xx[i] = make_float2(__uint_as_float(__float_as_uint(xx[i].x) ^ sg),
-                                  __uint_as_float(__float_as_uint(xx[i].y) ^ sg));
+              const float2 c = cmulf(cth, make_float2(x[i], y[i]));
+              x[i] = c.x;
+              y[i] = c.y;
             }
-          }
-          // A row (this lane): K = row (real parts) and 32 + row (imaginary parts), two bf16 per
-          // column, so rows 8q .. 8q+7 are columns 4q .. 4q+3 (re) and 16 + the same (im)
-          uint32_t hr[4], lr[4], hm[4], lm[4];
+            uint32_t hr[4], lr[4], hm[4], lm[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 a = xx[2 * i], c = xx[2 * i + 1];
-            hr[i] = pack_bf16(a.x, c.x);
-            hm[i] = pack_bf16(a.y, c.y);
-            lr[i] = pack_bf16(a.x - lo_half(hr[i]), c.x - hi_half(hr[i]));
-            lm[i] = pack_bf16(a.y - lo_half(hm[i]), c.y - hi_half(hm[i]));
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t wr = pack_bf16(x[2 * i], x[2 * i + 1]), wm = pack_bf16(y[2 * i], y[2 * i + 1]);
+              hr[i] = wr ^ mp[i] ^ m4[q];
+              hm[i] = wm ^ mp[i] ^ m4[q];
+              lr[i] = pack_neg_residual(wr, x[2 * i], x[2 * i + 1]) ^ mp[i] ^ m4[q];
+              lm[i] = pack_neg_residual(wm, y[2 * i], y[2 * i + 1]) ^ mp[i] ^ m4[q];
+            }
+            tmem_st4(taddr_a + uint32_t(4 * q), hr);
+            tmem_st4(taddr_a + uint32_t(16 + 4 * q), hm);
+            tmem_st4(taddr_a + uint32_t(32 + 4 * q), lr);
+            tmem_st4(taddr_a + uint32_t(48 + 4 * q), lm);
           }
-          tmem_st4(taddr_a + uint32_t(4 * q), hr);
-          tmem_st4(taddr_a + uint32_t(16 + 4 * q), hm);
-          tmem_st4(taddr_a + uint32_t(32 + 4 * q), lr);
-          tmem_st4(taddr_a + uint32_t(48 + 4 * q), lm);
+        } else if (flip) {
+          uint32_t mp[4], m4[4];
+          sign_pairs(par, mp, m4);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            float x[8], y[8];  // rows 8q..8q+7, loaded before any other work
+#pragma unroll
+            for (int i = 0; i < 8; ++i) lds_amp(lo8[i] ^ hi4[q], x[i], y[i]);
+            uint32_t hr[4], lr[4], hm[4], lm[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t wr = pack_bf16(x[2 * i], x[2 * i + 1]), wm = pack_bf16(y[2 * i], y[2 * i + 1]);
+              hr[i] = wr ^ mp[i] ^ m4[q];
+              hm[i] = wm ^ mp[i] ^ m4[q];
+              lr[i] = pack_neg_residual(wr, x[2 * i], x[2 * i + 1]) ^ mp[i] ^ m4[q];
+              lm[i] = pack_neg_residual(wm, y[2 * i], y[2 * i + 1]) ^ mp[i] ^ m4[q];
+            }
+            tmem_st4(taddr_a + uint32_t(4 * q), hr);
+            tmem_st4(taddr_a + uint32_t(16 + 4 * q), hm);
+            tmem_st4(taddr_a + uint32_t(32 + 4 * q), lr);
+            tmem_st4(taddr_a + uint32_t(48 + 4 * q), lm);
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            float x[8], y[8];  // rows 8q..8q+7, loaded before any other work
+#pragma unroll
+            for (int i = 0; i < 8; ++i) lds_amp(lo8[i] ^ hi4[q], x[i], y[i]);
+            uint32_t hr[4], lr[4], hm[4], lm[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              hr[i] = pack_bf16(x[2 * i], x[2 * i + 1]);
+              hm[i] = pack_bf16(y[2 * i], y[2 * i + 1]);
+              lr[i] = pack_neg_residual(hr[i], x[2 * i], x[2 * i + 1]);
+              lm[i] = pack_neg_residual(hm[i], y[2 * i], y[2 * i + 1]);
+            }
+            tmem_st4(taddr_a + uint32_t(4 * q), hr);
+            tmem_st4(taddr_a + uint32_t(16 + 4 * q), hm);
+            tmem_st4(taddr_a + uint32_t(32 + 4 * q), lr);
+            tmem_st4(taddr_a + uint32_t(48 + 4 * q), lm);
+          }
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
-        if (bar_any(1 + g, GROUP_THREADS, abort_sh)) break;
-        if (tg == 0) {
-          if (!mbar_wait(bar_ofull(sl), uint32_t((k / NOPSLOT) & 1))) fail(2);
+        bar_group(g);
+        if ((warp & 3) == 0) {
+          // all four warps' splits are in TMEM, the operand is in its slot (on a timeout the
+          // MMAs read stale operands and the group stops at its next barrier)
+          if (!mbar_wait(bar_ofull(sl), sl_phase)) fail(2);
+          __syncwarp();
           tc_fence_after();
-          const uint32_t b_hi = smem_u32(smem + SM_B + sl * OPERAND_BYTES);
-          const uint32_t b_lo = b_hi + OPERAND_BYTES / 2;
-          const uint64_t dbh = sw128_desc(b_hi), dbl = sw128_desc(b_lo);
-          // K = 16 per MMA: eight A columns, two 16-byte steps of B
+          const uint32_t slu = __shfl_sync(0xffffffffu, sl, 0);
+          const uint32_t b_hi = slot_addr(slu);
+          const uint64_t dbh = sw128_desc(b_hi), dbl = sw128_desc(b_hi + OPERAND_BYTES / 2);
+          if (elect_one()) {  // K = 16 per MMA: eight A columns, two 16-byte steps of B
 #pragma unroll
-          for (int s = 0; s < 4; ++s) mma_bf16_ta(d_tmem, a_tmem + 8u * s, dbh + 2 * s, idesc, s > 0);
+            for (int s = 0; s < 4; ++s) mma_bf16_ta(d_tmem, a_tmem + 8u * s, dbh + 2 * s, idesc, s > 0);
 #pragma unroll
-          for (int s = 0; s < 4; ++s) mma_bf16_ta(d_tmem, a_tmem + 32u + 8u * s, dbh + 2 * s, idesc, 1);
+            for (int s = 0; s < 4; ++s) mma_bf16_ta(d_tmem, a_tmem + 32u + 8u * s, dbh + 2 * s, idesc | NEGATE_A, 1);
 #pragma unroll
-          for (int s = 0; s < 4; ++s) mma_bf16_ta(d_tmem, a_tmem + 8u * s, dbl + 2 * s, idesc, 1);
-          mma_commit(bar_mma(g));
-          mma_commit(bar_oempty(sl));  // the slot is free once these MMAs have read it
+            for (int s = 0; s < 4; ++s) mma_bf16_ta(d_tmem, a_tmem + 8u * s, dbl + 2 * s, idesc, 1);
+            mma_commit(bar_mma(gu));
+            mma_commit(bar_oempty(slu));  // the slot is free once these MMAs have read it
+          }
+          __syncwarp();
         }
+        if (++sl == NOPSLOT) sl = 0, sl_phase ^= 1u;
         // a following diagonal op, reduced to this column (computed while the MMAs run)
-        uint32_t smask2 = 0;
-        float2 cth2 = make_float2(1.f, 0.f);
-        bool scal2 = false;
-        column_chunks(s_chunks, act_sh[g], op.qc0, op.qc1, uint32_t(tg), s_terms, smask2, cth2, scal2);
-        scal2 = __any_sync(0xffffffffu, scal2);
-        const bool flip2 = __any_sync(0xffffffffu, smask2 != 0);
+        uint32_t par2 = 0;
+        cth = make_float2(1.f, 0.f);
+        scal = false;
+        column_chunks(S.chunks, act, tph, op.qc0, op.qc1, uint32_t(tg), S.terms.coef, par2, cth, scal);
+        scal = __any_sync(0xffffffffu, scal);
+        const bool flip2 = __any_sync(0xffffffffu, par2 != 0);
         // every thread waits for the accumulator itself (no group barrier: each warp reads its
-        // lanes back as soon as the MMAs land).  A phase cannot be skipped: the next commit
-        // needs every warp past the barrier after this read-back.  On a timeout the read-back
-        // reads stale columns and the barrier below stops the group.
+        // lanes back as soon as the MMAs land).  A phase cannot be skipped: the next one needs
+        // every warp's split after this read-back.  On a timeout the read-back reads stale
+        // columns and the group stops at its next barrier.
         if (!mbar_wait(bar_mma(g), mma_phase)) fail(2);
         mma_phase ^= 1u;
         tc_fence_after();
-        // D columns 16h .. 16h+15 hold rows 8h .. 8h+7 as (real, imaginary) pairs
+        // D columns 16h .. 16h+15 hold rows 8h .. 8h+7 as (real, imaginary) pairs.  Two loops: in one,
+        // results kept in place past a branch cost a register copy each (72 an op).
+        if (!scal && !flip2) {
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          uint32_t v[16];
-          NCSIM_TMEM_LD16(taddr + uint32_t(16 * h), v);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (scal2) {
+          for (int h = 0; h < 4; ++h) {
+            uint32_t v[16];
+            NCSIM_TMEM_LD16(taddr + uint32_t(16 * h), v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sts_amp(lo8[i] ^ hi4[h], v[2 * i], v[2 * i + 1]);
+          }
+        } else {
+          uint32_t m8[8], m4[4];
+          sign_words(par2, m8, m4);
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            uint32_t v[16];
+            NCSIM_TMEM_LD16(taddr + uint32_t(16 * h), v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              const float2 c = cmulf(cth2, make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
-              v[2 * i] = __float_as_uint(c.x);
-              v[2 * i + 1] = __float_as_uint(c.y);
+              const float2 c = cmulf(cth, make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+              sts_amp(lo8[i] ^ hi4[h], __float_as_uint(c.x) ^ m8[i] ^ m4[h], __float_as_uint(c.y) ^ m8[i] ^ m4[h]);
             }
           }
-          if (flip2) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const uint32_t sg = (smask2 << (31 - (8 * h + i))) & 0x80000000u;
-              v[2 * i] ^= sg;
-              v[2 * i + 1] ^= sg;
-            }
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            T[lo8[i] ^ hi4[h]] = make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
         }
         tc_fence_before();
-        if (bar_any(1 + g, GROUP_THREADS, abort_sh)) break;
       }
-      if (bar_any(1 + g, GROUP_THREADS, abort_sh)) break;
-      if (mine) {
-        // the group writes its tile back; each thread's shared-memory reads are done once its
-        // stores are issued, so the buffer is free for the next load after every thread arrives
-        const float4* buf = reinterpret_cast<const float4*>(T);
-#pragma unroll 4
-        for (uint32_t c = uint32_t(tg); c < uint32_t(TILE) / 2; c += GROUP_THREADS)
-          *reinterpret_cast<float4*>(chunk_addr(base, c)) = buf[at(2u * c) >> 1];
-        mbar_arrive(bar_tdone(b));
+      if (stop || bar_any(1 + g, GROUP_THREADS, S.abort)) break;
+      // the group writes its tile back; each thread's shared-memory reads are done once its
+      // stores are issued, so the buffer is free for the next load after every warp arrives
+      uint8_t* const dst = reinterpret_cast<uint8_t*>(P.amp) + base * sizeof(float2) + my_off;
+      const uint32_t src = (tiles0 + b * TILE_BYTES) ^ my_at;
+#pragma unroll
+      for (uint32_t i = 0; i < uint32_t(TILE / 2 / GROUP_THREADS); ++i) {
+        const uint32_t e = 2u * GROUP_THREADS * i;
+        float4 v;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                     : "r"(src ^ (8u * (e ^ swz_fold(e)))));
+        *reinterpret_cast<float4*>(dst + S.chunk_off[GROUP_THREADS / TILE_THREADS * i]) = v;
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_tdone(b));
+      b += NG;
+      if (b >= NTILEBUF) b -= NTILEBUF, parity ^= 1u;
     }
   }
   tc_fence_before();
@@ -693,11 +843,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused_pass(const __grid_constant
 // device copy of a plan: every pass's operand images in one buffer
 struct DevicePlan {
   Plan plan;
-  std::vector<PassParams> params;  // per pass, in segment order (amp/err filled per run)
-  uint8_t* rops = nullptr;
+  std::vector<PassArgs> args;  // per pass, in segment order (amp/err filled per run)
+  uint8_t* images = nullptr;   // the operands, then the passes' tables
   int device = -1;
   ~DevicePlan() {
-    if (rops) cudaFree(rops);
+    if (images) cudaFree(images);
   }
 };
 
@@ -710,22 +860,81 @@ TermClass term_class(uint32_t tm, const CplxD& c) {
   return T_GENERIC;
 }
 
+// The order of a unitary's column bits.  A warp access moves its amplitudes 16 lanes (8 bytes each)
+// at a time, and each lane's bank is linear in the tile bits (a low bit's own, a higher bit's fold):
+// there are no conflicts when the four lowest column bits have independent banks.  They are picked
+// greedily, the rest follow.  Over the layered circuits' plans (195 unitaries) a warp access takes
+// 2.35 wavefronts instead of 2.46 with the bits in ascending order; 2 is the minimum, and the
+// unitaries on tile bit 0, whose bank no other bit reaches, take 4.
+void column_order(const uint8_t (&pos)[GROUP_QUBITS], uint8_t (&col)[COL_BITS]) {
+  uint32_t gm = 0;
+  for (uint8_t p : pos) gm |= 1u << p;
+  uint32_t span = 1;     // bank vectors (4 bits) reachable by the picked bits, as a set
+  uint32_t picked = 0;
+  int m = 0;
+  for (int b = 0; b < TILE_BITS && m < 4; ++b) {
+    if ((gm >> b) & 1) continue;
+    const uint32_t v = (b < 4 ? 1u << b : swz_fold(1u << b)) & 15u;
+    if ((span >> v) & 1) continue;
+    uint32_t next = span;
+    for (uint32_t x = 0; x < 16; ++x)
+      if ((span >> x) & 1) next |= 1u << (x ^ v);
+    span = next;
+    picked |= 1u << b;
+    col[m++] = uint8_t(b);
+  }
+  for (int b = 0; b < TILE_BITS; ++b)
+    if (!(((gm | picked) >> b) & 1)) col[m++] = uint8_t(b);
+}
+
+PassTables build_tables(const PassProgram& P, const std::vector<uint32_t>& window) {
+  PassTables T{};
+  std::copy(P.chunks, P.chunks + P.nchunks, T.chunks);
+  std::copy(P.ops, P.ops + P.nops, T.ops);
+  for (int i = 0; i < P.nterms; ++i) {
+    T.terms.cmask[i] = P.terms[i].cmask;
+    T.terms.coef[i] = make_float2(P.terms[i].cr, P.terms[i].ci);
+    T.terms.tmask[i] = uint16_t(P.terms[i].tmask);
+  }
+  auto stored = [](uint32_t e) { return uint16_t((e ^ swz_fold(e)) * sizeof(float2)); };
+  for (int u = 0; u < P.nu; ++u) {
+    auto column = [&](uint32_t k) {
+      uint32_t e = 0;
+      for (int m = 0; m < COL_BITS; ++m) e |= ((k >> m) & 1u) << P.col[u][m];
+      return stored(e);
+    };
+    for (uint32_t k = 0; k < 16; ++k) T.clo[u][k] = column(k);
+    for (uint32_t k = 0; k < 8; ++k) T.chi[u][k] = column(k << 4);
+    for (int j = 0; j < GROUP_QUBITS; ++j) T.gbit[u][j] = stored(1u << P.pos[u][j]);
+  }
+  for (uint32_t i = 0; i < uint32_t(TILE / 2 / TILE_THREADS); ++i) {
+    const uint32_t e = 2u * TILE_THREADS * i;
+    for (int j = 0; j < TILE_BITS; ++j) T.chunk_off[i] |= (uint64_t((e >> j) & 1u) << window[j]) * sizeof(float2);
+  }
+  for (uint32_t h = 0; h < (1u << (TILE_BITS - 4)); ++h) T.swz[h] = uint8_t(swz_fold(h << 4));
+  for (int j = 0; j < TILE_BITS; ++j) T.win[j] = uint8_t(window[j]);
+  for (uint32_t q = 0, j = 0, m = 0; m < 32; ++q) {  // the index bits outside the window
+    if (j < uint32_t(TILE_BITS) && window[j] == q) ++j;
+    else T.out[m++] = uint8_t(q);
+  }
+  return T;
+}
+
 std::unique_ptr<DevicePlan> build_device_plan(const ncsim_circuit& c, uint32_t max_fuse, cudaStream_t stream) {
   auto dp = std::make_unique<DevicePlan>();
   dp->plan = make_plan(c, max_fuse);
   std::vector<uint8_t> images;
   std::vector<size_t> offsets;
+  std::vector<PassTables> tables;
   for (const Segment& s : dp->plan.segments) {
     if (!s.fused) continue;
     for (const Pass& ps : s.passes) {
-      PassParams P{};
-      P.ntiles = (uint64_t(1) << c.n) >> TILE_BITS;
+      PassProgram P{};
       uint64_t wmask = 0;
-      for (int j = 0; j < TILE_BITS; ++j) P.win[j] = uint8_t(ps.window[j]), wmask |= uint64_t(1) << ps.window[j];
+      for (int j = 0; j < TILE_BITS; ++j) wmask |= uint64_t(1) << ps.window[j];
       int wl = 0;
       while (wl < TILE_BITS && ps.window[wl] == uint32_t(wl)) ++wl;
       if (wl < LOW_BITS) throw Error(NCSIM_ERR_INVALID, "fused pass window lacks the low index bits");
-      P.wl = wl;
       int nu = 0, nt = 0, no = 0;
       for (const FusedOp& op : ps.ops) {
         OpDesc d{};
@@ -738,6 +947,7 @@ std::unique_ptr<DevicePlan> build_device_plan(const ncsim_circuit& c, uint32_t m
             if (it == ps.window.end()) throw Error(NCSIM_ERR_INVALID, "fused unitary outside its window");
             P.pos[nu][j] = uint8_t(it - ps.window.begin());
           }
+          column_order(P.pos[nu], P.col[nu]);
           const size_t at = images.size();
           images.resize(at + OPERAND_BYTES);
           build_operand_image(op.u, images.data() + at);
@@ -782,7 +992,6 @@ std::unique_ptr<DevicePlan> build_device_plan(const ncsim_circuit& c, uint32_t m
       // qubits, phases of the other bits or signs on one of its qubits is applied while the
       // unitary splits the tile (kind 2); one left after a unitary, by its read-back (kind 3).
       // Their terms go to the device as chunks of bit masks over 32 terms.
-      static const uint32_t rowpat[GROUP_QUBITS] = {0xAAAAAAAAu, 0xCCCCCCCCu, 0xF0F0F0F0u, 0xFF00FF00u, 0xFFFF0000u};
       int nch = 0;
       auto fold = [&](OpDesc& t, OpDesc& un, uint8_t kind) -> bool {
         uint32_t gm = 0;
@@ -795,7 +1004,8 @@ std::unique_ptr<DevicePlan> build_device_plan(const ncsim_circuit& c, uint32_t m
         const int need = (t.t1 - t.t0 + 31) / 32;
         if (nch + need > MAX_CHUNKS) return false;
         int colbit[TILE_BITS];  // tile bit -> column bit of this unitary (-1: a gate bit)
-        for (int b = 0, m = 0; b < TILE_BITS; ++b) colbit[b] = ((gm >> b) & 1) ? -1 : m++;
+        for (int& cb : colbit) cb = -1;
+        for (int m = 0; m < COL_BITS; ++m) colbit[P.col[un.u][m]] = m;
         const uint8_t c0 = uint8_t(nch);
         for (int k0 = t.t0; k0 < t.t1; k0 += 32) {
           ColChunk ch{};
@@ -805,14 +1015,15 @@ std::unique_ptr<DevicePlan> build_device_plan(const ncsim_circuit& c, uint32_t m
             TermDesc& td = P.terms[k0 + i];
             const uint32_t bit = 1u << i;
             const uint32_t gpart = td.tmask & gm;
-            td.rowpat = 0;
+            bool rows = false;
             for (int j = 0; j < GROUP_QUBITS; ++j)
-              if (gpart == (1u << P.pos[un.u][j])) td.rowpat = rowpat[j], ch.row[j] |= bit;
+              if (gpart == (1u << P.pos[un.u][j])) rows = true, ch.row[j] |= bit;
             td.tmask &= ~gm;
             for (int b = 0; b < TILE_BITS; ++b)
               if ((td.tmask >> b) & 1) ch.need[colbit[b]] |= bit;
-            if (!td.rowpat) {
+            if (!rows) {
               if (td.cr == -1.0f && td.ci == 0.0f) ch.neg |= bit;
+              else if (td.tmask == 0 && k0 == t.t0 && !ch.gen) ch.tgen |= bit;
               else ch.gen |= bit;
             }
           }
@@ -828,19 +1039,33 @@ std::unique_ptr<DevicePlan> build_device_plan(const ncsim_circuit& c, uint32_t m
       for (int i = 1; i < no; ++i)
         if (P.ops[i].kind == 1 && P.ops[i - 1].kind == 0) fold(P.ops[i], P.ops[i - 1], 3);
       P.nchunks = nch;
+      P.nterms = nt;
+      P.nops = int(std::remove_if(P.ops, P.ops + no, [](const OpDesc& d) { return d.kind >= 2; }) - P.ops);
+      tables.push_back(build_tables(P, ps.window));
+      PassArgs a{};
+      a.ntiles = uint32_t((uint64_t(1) << c.n) >> TILE_BITS);
+      a.nops = P.nops;
+      a.nu = P.nu;
+      a.nchunks = P.nchunks;
       // the pass's first operand: an offset for now, a device pointer below
-      P.rops = reinterpret_cast<const uint4*>(uintptr_t(nu ? offsets[offsets.size() - nu] : 0));
-      dp->params.push_back(P);
+      a.rops = reinterpret_cast<const uint4*>(uintptr_t(nu ? offsets[offsets.size() - nu] : 0));
+      dp->args.push_back(a);
     }
   }
+  const size_t at = images.size();
+  images.resize(at + tables.size() * sizeof(PassTables));
   if (!images.empty()) {
-    NCSIM_CUDA(cudaMalloc(&dp->rops, images.size()));
+    if (!tables.empty()) std::memcpy(images.data() + at, tables.data(), tables.size() * sizeof(PassTables));
+    NCSIM_CUDA(cudaMalloc(&dp->images, images.size()));
     // on the state's stream, waited for: a pageable cudaMemcpy may return before its DMA lands,
     // and the pass kernels' non-blocking stream does not wait for the legacy stream
-    NCSIM_CUDA(cudaMemcpyAsync(dp->rops, images.data(), images.size(), cudaMemcpyHostToDevice, stream));
+    NCSIM_CUDA(cudaMemcpyAsync(dp->images, images.data(), images.size(), cudaMemcpyHostToDevice, stream));
     NCSIM_CUDA(cudaStreamSynchronize(stream));
   }
-  for (auto& P : dp->params) P.rops = reinterpret_cast<const uint4*>(dp->rops + uintptr_t(P.rops));
+  for (size_t i = 0; i < dp->args.size(); ++i) {
+    dp->args[i].rops = reinterpret_cast<const uint4*>(dp->images + uintptr_t(dp->args[i].rops));
+    dp->args[i].tables = reinterpret_cast<const PassTables*>(dp->images + at) + i;
+  }
   NCSIM_CUDA(cudaGetDevice(&dp->device));
   return dp;
 }
@@ -887,9 +1112,14 @@ extern "C" ncsim_status ncsim_sv_run_fused(ncsim_state* s, const ncsim_circuit* 
     std::shared_ptr<fused::DevicePlan> dp = device_plan_for(c, max_fuse ? max_fuse : 5, s->stream);
     int* d_err = s->dev_flag;  // the state's own word: no allocation per run
     NCSIM_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), s->stream));
-    NCSIM_CUDA(cudaFuncSetAttribute(fused::k_fused_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, fused::SM_DYNAMIC));
-    const uint64_t sets = ((s->len >> fused::TILE_BITS) + fused::GROUPS - 1) / fused::GROUPS;  // a tile per warpgroup
-    const unsigned grid = unsigned(std::min<uint64_t>(uint64_t(sm_count()), sets));
+    // A tile per warpgroup; a register of fewer tiles than four per SM spreads them first, since
+    // groups of one CTA share its tensor core and shared memory: n = 16
+    // 94 -> 69 us, n = 19 109 -> 80, n = 20 120 -> 97 against four tiles to a CTA.
+    const uint64_t ntiles = s->len >> fused::TILE_BITS, sms = uint64_t(sm_count());
+    const uint64_t groups = ntiles <= sms ? 1 : ntiles <= 2 * sms ? 2 : fused::GROUPS;
+    const unsigned grid = unsigned(std::min<uint64_t>(sms, (ntiles + groups - 1) / groups));
+    const auto kernel = groups == 1 ? fused::k_fused_pass<1> : groups == 2 ? fused::k_fused_pass<2> : fused::k_fused_pass<4>;
+    NCSIM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fused::SM_DYNAMIC));
     size_t m = 0, pi = 0;
     uint64_t gemm = 0;
     for (const fused::Segment& seg : dp->plan.segments) {
@@ -899,12 +1129,12 @@ extern "C" ncsim_status ncsim_sv_run_fused(ncsim_state* s, const ncsim_circuit* 
         continue;
       }
       for (size_t k = 0; k < seg.passes.size(); ++k, ++pi) {
-        fused::PassParams P = dp->params[pi];
+        fused::PassArgs P = dp->args[pi];
         P.amp = reinterpret_cast<float2*>(s->amp);
         P.err = d_err;
         ++gemm;  // one pass kernel launch
         ProfScope ps(s, K_FUSED_GEMM, 2.0 * double(s->bytes()));
-        fused::k_fused_pass<<<grid, fused::THREADS, fused::SM_DYNAMIC, s->stream>>>(P);
+        kernel<<<grid, fused::THREADS, fused::SM_DYNAMIC, s->stream>>>(P);
         NCSIM_LAUNCHED("fused pass");
       }
     }
