@@ -33,7 +33,6 @@
 #include <cmath>
 #include <map>
 #include <numeric>
-#include <queue>
 #include <thread>
 
 #include <sys/stat.h>
@@ -889,46 +888,68 @@ struct LaunchShape {
   }
 };
 
+// How many clusters of C CTAs the device holds at once (0: none): asked once per device and kernel,
+// the query takes as long as a small batch's launch.
+uint32_t resident_clusters(const ncsim_batch_config& cfg, uint32_t C, cudaStream_t st) {
+  constexpr int DEVICES = 64;
+  static std::atomic<int> known[DEVICES][2][4];  // the answer plus one
+  int dev = 0;
+  NCSIM_CUDA(cudaGetDevice(&dev));
+  std::atomic<int>* const memo = dev < DEVICES ? &known[dev][cfg.buffers == 1][__builtin_ctz(C)] : nullptr;
+  int fit = memo ? memo->load() - 1 : -1;
+  if (fit < 0) {
+    LaunchShape l(cfg, C, grid_for(cfg) / C * C, st);
+    const cudaError_t e = cfg.buffers == 1 ? cudaOccupancyMaxActiveClusters(&fit, k_batch<1, true>, &l.config)
+                                           : cudaOccupancyMaxActiveClusters(&fit, k_batch<2, true>, &l.config);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    if (memo) memo->store(fit + 1);
+  }
+  return uint32_t(fit);
+}
+
 // CTAs per trajectory: the C whose schedule ends first.  Trajectories go to the clusters in order, each
-// to the one that is free first; a trajectory takes ceil(tiles / C) tile times and half a tile time (the
-// pass's descriptors, pipeline fill and barrier) per pass.  A larger C must end 4% earlier: its clusters
-// leave SMs of a GPC unused, and more CTAs share each pass's fixed part.
+// to the one that is free first; a trajectory takes ceil(tiles / C) tile times and a fixed part per pass:
+// half a tile time for one CTA (the pass's descriptors, pipeline fill and barrier), one and a quarter for
+// a cluster (its barriers as well; fitted to 14 to 16 qubits, where a cluster's pass is a few tiles: 508
+// trajectories of 15 qubits 752 us with C = 1 and 780 with 2, of 13 to 15 414 and 511, 148 of 14 168 and
+// 155, of 16 634, 465 and with C = 4 570).  A larger C must end 4% earlier: its clusters leave SMs of a GPC
+// unused, and more CTAs share each pass's fixed part.
 uint32_t cluster_size(const ncsim_batch* b, const ncsim_batch_config& cfg, const std::vector<uint32_t>& order,
                       uint32_t* clusters) {
-  uint32_t best = 1;
+  uint32_t best = 1, tiles_max = 1;
   double best_end = 0.0;
-  for (uint32_t C = 1; C <= 8; C *= 2) {
+  for (uint32_t t : order) tiles_max = std::max(tiles_max, 1u << (b->prog.traj[t].n - TILE_BITS));
+  std::vector<double> free_at;  // a heap, the first free on top
+  for (uint32_t C = 1; C <= 8 && C <= tiles_max; C *= 2) {
     uint32_t servers = grid_for(cfg);
-    if (C > 1) {
-      LaunchShape l(cfg, C, servers / C * C, b->stream);
-      int fit = 0;
-      const cudaError_t e = cfg.buffers == 1 ? cudaOccupancyMaxActiveClusters(&fit, k_batch<1, true>, &l.config)
-                                             : cudaOccupancyMaxActiveClusters(&fit, k_batch<2, true>, &l.config);
-      if (e != cudaSuccess || fit < 1) {
-        cudaGetLastError();
-        continue;
-      }
-      servers = std::min(uint32_t(fit), servers / C);
-    }
-    std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
-    double end = 0.0;
+    if (C > 1) servers = std::min(resident_clusters(cfg, C, b->stream), servers / C);
+    if (!servers) continue;
+    free_at.assign(std::min<size_t>(servers, order.size()), 0.0);
+    double end = 0.0, busy = 0.0;
     for (uint32_t t : order) {
-      double at = 0.0;
-      if (free_at.size() >= servers) {
-        at = free_at.top();
-        free_at.pop();
-      }
       const DevTraj& tr = b->prog.traj[t];
-      const double tiles = double((1u << (tr.n - TILE_BITS)) + C - 1) / C;
-      at += tr.npass * (std::floor(tiles) + 0.5);
+      const uint32_t tiles = ((1u << (tr.n - TILE_BITS)) + C - 1) / C;
+      const double takes = tr.npass * (double(tiles) + (C == 1 ? 0.5 : 1.25)), at = free_at[0] + takes;
+      busy += takes;
       end = std::max(end, at);
-      free_at.push(at);
+      size_t i = 0;  // the new time sinks to its place
+      for (size_t c = 1; c < free_at.size(); i = c, c = 2 * i + 1) {
+        if (c + 1 < free_at.size() && free_at[c + 1] < free_at[c]) ++c;
+        if (free_at[c] >= at) break;
+        free_at[i] = free_at[c];
+      }
+      free_at[i] = at;
     }
     if (C == 1 || end < 0.96 * best_end) {
       best = C;
       best_end = end;
       *clusters = servers;
     }
+    // no C ends before the whole work shared evenly
+    if (C == 1 && busy / servers >= 0.96 * end) break;
   }
   return best;
 }
