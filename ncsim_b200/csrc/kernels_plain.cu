@@ -600,9 +600,18 @@ __global__ void __launch_bounds__(THREADS) k_pauli_pair(V<R>* __restrict__ a, ui
   }
 }
 
+// The kernels of a measurement may launch under the end of the kernel before them (launch_measure):
+// they touch nothing before that one is done.  Each takes 2 to 5 us at 17 qubits and waited as long for its
+// launch: a noisy trajectory with 48 measurements 1050 -> 888 us; n = 6 710 -> 583, n = 20 1633 -> 1467,
+// n = 22 and above within 3% (faster).
+__device__ __forceinline__ void after_previous_kernel() {
+  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+
 // X on bit h when the measurement before it came out 1 (a reset's flip)
 template <class R>
 __global__ void __launch_bounds__(THREADS) k_flip_if(V<R>* __restrict__ a, uint64_t npairs, int h, const int* decided) {
+  after_previous_kernel();
   if (!*decided) return;
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   const uint64_t lo = (uint64_t(1) << h) - 1;
@@ -776,6 +785,7 @@ __device__ void decide_in_last_block(const double* partials, MeasureQueue* q, in
 template <class R, bool NORM>
 __global__ void __launch_bounds__(REDUCE_THREADS) k_expect_diag(const V<R>* __restrict__ a, uint64_t len, uint64_t z, int ph,
                                                                 double* partials, MeasureQueue* queue = nullptr, int slot = 0) {
+  after_previous_kernel();
   // sum_c i^{k(c)} |psi(c)|^2
   double acc[3] = {0.0, 0.0, 0.0};
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
@@ -802,6 +812,7 @@ template <class R, bool NORM>
 __global__ void __launch_bounds__(REDUCE_THREADS) k_expect_pair(const V<R>* __restrict__ a, uint64_t npairs, int h, uint64_t x,
                                                                 uint64_t z, int ph, double* partials,
                                                                 MeasureQueue* queue = nullptr, int slot = 0) {
+  after_previous_kernel();
   double acc[3] = {0.0, 0.0, 0.0};
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   const uint64_t lo = (uint64_t(1) << h) - 1;
@@ -890,6 +901,7 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_compare(const V<RA>* __restr
 template <class R>
 __global__ void __launch_bounds__(REDUCE_THREADS) k_project_diag(V<R>* __restrict__ a, uint64_t len, uint64_t z, int ph, int outcome,
                                                                  double* partials, const int* decided = nullptr) {
+  after_previous_kernel();
   if (decided) outcome = *decided;  // a measurement's, taken on the device
   double acc[1] = {0.0};
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
@@ -916,6 +928,7 @@ template <class R>
 __global__ void __launch_bounds__(REDUCE_THREADS) k_project_pair(V<R>* __restrict__ a, uint64_t npairs, int h, uint64_t x, uint64_t z,
                                                                  int ph, int outcome, double* partials,
                                                                  const int* decided = nullptr) {
+  after_previous_kernel();
   if (decided) outcome = *decided;
   double acc[1] = {0.0};
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
@@ -1589,6 +1602,21 @@ int launch_project_partials(ncsim_state* s, uint64_t x, uint64_t z, uint32_t pha
 bool can_measure_on_device(const ncsim_state* s) { return reduce_grid(s->len) <= DECIDE_BLOCKS; }
 
 // measurement `slot` of the queue: outcome and projection, nothing waited for; a reset also flips on 1
+// a kernel that calls after_previous_kernel first, launched under the end of the stream's last kernel
+template <class... P, class... A>
+static void launch_under(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute overlap{};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t launch{};
+  launch.gridDim = dim3(grid);
+  launch.blockDim = dim3(block);
+  launch.stream = stream;
+  launch.attrs = &overlap;
+  launch.numAttrs = 1;
+  NCSIM_CUDA(cudaLaunchKernelEx(&launch, kernel, P(args)...));
+}
+
 void launch_measure(ncsim_state* s, uint64_t x, uint64_t z, uint32_t phase, MeasureQueue* queue, int slot, bool reset) {
   const int ph = int(phase & 3);
   const int* decided = &queue->outcome[slot];
@@ -1597,25 +1625,25 @@ void launch_measure(ncsim_state* s, uint64_t x, uint64_t z, uint32_t phase, Meas
       const int g = reduce_grid(s->len);
       {
         ProfScope ps(s, K_EXPECT, 0.5 * full_bytes(s));
-        k_expect_diag<R, true><<<g, REDUCE_THREADS, 0, s->stream>>>(amp_of<R>(s), s->len, z, ph, s->partials, queue, slot);
+        launch_under(k_expect_diag<R, true>, g, REDUCE_THREADS, s->stream, amp_of<R>(s), s->len, z, ph, s->partials, queue, slot);
       }
       ProfScope ps(s, K_PROJECT, 0.5 * full_bytes(s));
-      k_project_diag<R><<<g, REDUCE_THREADS, 0, s->stream>>>(amp_of<R>(s), s->len, z, ph, 0, s->partials, decided);
+      launch_under(k_project_diag<R>, g, REDUCE_THREADS, s->stream, amp_of<R>(s), s->len, z, ph, 0, s->partials, decided);
     } else {
       const int h = 63 - __builtin_clzll(x);
       const uint64_t np = s->len >> 1;
       const int g = reduce_grid(np);
       {
         ProfScope ps(s, K_EXPECT, 0.5 * full_bytes(s));
-        k_expect_pair<R, true><<<g, REDUCE_THREADS, 0, s->stream>>>(amp_of<R>(s), np, h, x, z, ph, s->partials, queue, slot);
+        launch_under(k_expect_pair<R, true>, g, REDUCE_THREADS, s->stream, amp_of<R>(s), np, h, x, z, ph, s->partials, queue, slot);
       }
       ProfScope ps(s, K_PROJECT, full_bytes(s));
-      k_project_pair<R><<<g, REDUCE_THREADS, 0, s->stream>>>(amp_of<R>(s), np, h, x, z, ph, 0, s->partials, decided);
+      launch_under(k_project_pair<R>, g, REDUCE_THREADS, s->stream, amp_of<R>(s), np, h, x, z, ph, 0, s->partials, decided);
     }
     if (reset) {
       ProfScope ps(s, K_PAULI, full_bytes(s));
       const uint64_t np = s->len >> 1;
-      k_flip_if<R><<<grid_for(np, THREADS), THREADS, 0, s->stream>>>(amp_of<R>(s), np, 63 - __builtin_clzll(z), decided);
+      launch_under(k_flip_if<R>, grid_for(np, THREADS), THREADS, s->stream, amp_of<R>(s), np, 63 - __builtin_clzll(z), decided);
     }
   });
   NCSIM_LAUNCHED("measure");
