@@ -13,9 +13,14 @@
 //   key with bit 1:  S1[pair] + S0[end of the range].
 // A pair's sum has two terms, so it has the same bits in either order.
 //
+// Which outputs are kept is decided once, by the counting step; the placing step reads
+// that decision, so that an output never lands in a place that was not counted for it.
+// The values are made twice with the same fixed roundings.
+//
 // Up to SMALL_OUT outputs one block walks a whole list of gates (the Hadamards that open
 // a circuit) with one launch and one wait: 6 us a gate (n = 31, small sets) to 11 (16-word keys), where the sort-based form
-// took eleven launches, a wait and some 80 us.  Larger states take four launches a gate.
+// took eleven launches, a wait and some 80 us.  Larger states take five launches a gate
+// (merge, count, the scan's two, place).
 #include "sparse_dense.hpp"
 
 #include "sparse_common.cuh"
@@ -124,32 +129,36 @@ __device__ __forceinline__ uint32_t merged_place(const uint64_t* key, uint32_t m
   return o + (i - mid) + (o < m && equals_at<W>(key, o, other) ? 1u : 0u);
 }
 
-// The pair whose first entry stands at merged place p: which outputs are kept (bit 0: the key with
-// bit q = 0, bit 1: the other; 0 at the second entry of a pair) and their values.
+// The outputs of the pair whose first entry stands at merged place p (out[r]: the key with bit q = r),
+// in a fixed sequence of roundings; false at the second entry of a pair, whose place has none.
 template <int W>
-__device__ __forceinline__ uint32_t pair_outputs(const uint64_t* key, const double2* amp, const uint32_t i, bool has_prev,
-                                                 uint32_t prev, bool has_next, uint32_t next, const OnBit<W>& B,
-                                                 const double2* g, double cut2, double2 (&out)[2]) {
+__device__ __forceinline__ bool pair_values(const uint64_t* key, const double2* amp, const uint32_t i, bool has_prev,
+                                            uint32_t prev, bool has_next, uint32_t next, const OnBit<W>& B,
+                                            const double2* g, double2 (&out)[2]) {
   const DKey<W> k = load_key<W>(key, i);
   const bool one = B.one(k);
   const DKey<W> other = B.with(k, !one);
-  if (one && has_prev && equals_at<W>(key, prev, other)) return 0;
+  if (one && has_prev && equals_at<W>(key, prev, other)) return false;
   const double2 v = amp[i];
   const uint32_t col = one ? 1u : 0u;
-  out[0] = zmul(g[col], v);
-  out[1] = zmul(g[2 + col], v);
+  out[0] = cmul(g[col], v);
+  out[1] = cmul(g[2 + col], v);
   if (!one && has_next && equals_at<W>(key, next, other)) {
     const double2 u = amp[next];
-    const double2 a = zmul(g[1], u), b = zmul(g[3], u);
-    out[0] = make_double2(out[0].x + a.x, out[0].y + a.y);
-    out[1] = make_double2(out[1].x + b.x, out[1].y + b.y);
+    const double2 a = cmul(g[1], u), b = cmul(g[3], u);
+    out[0] = make_double2(__dadd_rn(out[0].x, a.x), __dadd_rn(out[0].y, a.y));
+    out[1] = make_double2(__dadd_rn(out[1].x, b.x), __dadd_rn(out[1].y, b.y));
   }
+  return true;
+}
+// which of a pair's outputs stay (bit r: out[r]): nonzero and not under the cutoff
+__device__ __forceinline__ uint32_t kept(const double2 (&out)[2], double cut2) {
   uint32_t keep = 0;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const double2 a = out[r];
     const bool zero = a.x == 0.0 && a.y == 0.0;
-    if (!zero && (cut2 == 0.0 || a.x * a.x + a.y * a.y >= cut2)) keep |= 1u << r;
+    if (!zero && (cut2 == 0.0 || __fma_rn(a.x, a.x, __dmul_rn(a.y, a.y)) >= cut2)) keep |= 1u << r;
   }
   return keep;
 }
@@ -186,13 +195,12 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_sp_dense1_small(const __grid_
     const uint32_t per = (m + SMALL_THREADS - 1) / SMALL_THREADS;
     const uint32_t p0 = min(threadIdx.x * per, m), p1 = min(p0 + per, m);
     const auto pair_at = [&](uint32_t p, double2 (&out)[2]) {
-      return pair_outputs<W>(key, amp, s_at[p], p > 0, s_at[p ? p - 1 : 0], p + 1 < m, s_at[p + 1 < m ? p + 1 : 0], B, g,
-                             P.cut2, out);
+      return pair_values<W>(key, amp, s_at[p], p > 0, s_at[p ? p - 1 : 0], p + 1 < m, s_at[p + 1 < m ? p + 1 : 0], B, g, out);
     };
     uint32_t mine = 0;
     double2 out[2];
     for (uint32_t p = p0; p < p1; ++p) {
-      const uint32_t keep = pair_at(p, out);
+      const uint32_t keep = pair_at(p, out) ? kept(out, P.cut2) : 0u;
       s_sum[p] = mine;  // within the range for now
       mine += (keep & 1u) | (keep >> 1) << 16;
     }
@@ -220,8 +228,10 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_sp_dense1_small(const __grid_
     for (uint32_t p = p0; p < p1; ++p) s_sum[p] += before;
     __syncthreads();
     for (uint32_t p = threadIdx.x; p < m; p += SMALL_THREADS) {
-      const uint32_t keep = pair_at(p, out);
+      const uint32_t counted = s_sum[p + 1] - s_sum[p];  // the counting step's decision
+      const uint32_t keep = (counted & 1u) | (counted >> 16) << 1;
       if (!keep) continue;
+      pair_at(p, out);
       const DKey<W> k = load_key<W>(key, s_at[p]);
       const uint32_t lo = lower_bound<W>(key, m, B.prefix(k, false));
       const DKey<W> end = B.last(k);
@@ -259,9 +269,9 @@ __global__ void k_sp_dense1_merge(const uint64_t* key, uint32_t m, uint32_t q, u
     at[merged_place<W>(key, m, uint32_t(i), B)] = uint32_t(i);
 }
 template <int W>
-__device__ __forceinline__ uint32_t pair_in(const uint64_t* key, const double2* amp, uint32_t m, const uint32_t* at, uint32_t p,
-                                            const OnBit<W>& B, const Gate1& g, double cut2, double2 (&out)[2]) {
-  return pair_outputs<W>(key, amp, at[p], p > 0, at[p ? p - 1 : 0], p + 1 < m, at[p + 1 < m ? p + 1 : 0], B, g.m, cut2, out);
+__device__ __forceinline__ bool pair_in(const uint64_t* key, const double2* amp, uint32_t m, const uint32_t* at, uint32_t p,
+                                        const OnBit<W>& B, const Gate1& g, double2 (&out)[2]) {
+  return pair_values<W>(key, amp, at[p], p > 0, at[p ? p - 1 : 0], p + 1 < m, at[p + 1 < m ? p + 1 : 0], B, g.m, out);
 }
 template <int W>
 __global__ void k_sp_dense1_count(const uint64_t* key, const double2* amp, uint32_t m, const uint32_t* at,
@@ -269,20 +279,22 @@ __global__ void k_sp_dense1_count(const uint64_t* key, const double2* amp, uint3
   const OnBit<W> B(g.q);
   for (uint64_t p = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; p <= m; p += uint64_t(gridDim.x) * blockDim.x) {
     double2 out[2];
-    const uint32_t keep = p < m ? pair_in<W>(key, amp, m, at, uint32_t(p), B, g, cut2, out) : 0u;
+    const uint32_t keep = p < m && pair_in<W>(key, amp, m, at, uint32_t(p), B, g, out) ? kept(out, cut2) : 0u;
     cnt[p] = uint64_t(keep & 1u) | uint64_t(keep >> 1) << 32;
   }
 }
 template <int W>
 __global__ void k_sp_dense1_place(const uint64_t* key, const double2* amp, uint32_t m, const uint32_t* at,
-                                  const __grid_constant__ Gate1 g, double cut2, const uint64_t* sum, uint64_t* okey,
+                                  const __grid_constant__ Gate1 g, const uint64_t* cnt, const uint64_t* sum, uint64_t* okey,
                                   double2* oamp, uint32_t* result) {
   const OnBit<W> B(g.q);
   for (uint64_t p = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < m; p += uint64_t(gridDim.x) * blockDim.x) {
-    double2 out[2];
-    const uint32_t keep = pair_in<W>(key, amp, m, at, uint32_t(p), B, g, cut2, out);
     if (p == 0) *result = uint32_t(sum[m]) + uint32_t(sum[m] >> 32);
+    const uint64_t counted = cnt[p];
+    const uint32_t keep = uint32_t(counted & 1u) | uint32_t(counted >> 32) << 1;
     if (!keep) continue;
+    double2 out[2];
+    pair_in<W>(key, amp, m, at, uint32_t(p), B, g, out);
     const DKey<W> k = load_key<W>(key, at[p]);
     const uint32_t lo = lower_bound<W>(key, m, B.prefix(k, false));
     const DKey<W> end = B.last(k);
@@ -377,7 +389,7 @@ void apply_large(ncsim_sparse* s, const SparseDense1& gate) {
   NCSIM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, sum, int(m + 1), st));
   void* tmp = dalloc<uint8_t>(tb, st);
   NCSIM_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, sum, int(m + 1), st));
-  k_sp_dense1_place<W><<<sp_grid(m), SP_THREADS, 0, st>>>(s->key, s->amp, uint32_t(m), at, g, cut2, sum, okey, oamp, result);
+  k_sp_dense1_place<W><<<sp_grid(m), SP_THREADS, 0, st>>>(s->key, s->amp, uint32_t(m), at, g, cnt, sum, okey, oamp, result);
   NCSIM_LAUNCHED("sparse dense gate (place)");
   dfree(tmp, st);
   dfree(at, st);
