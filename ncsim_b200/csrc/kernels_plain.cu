@@ -601,7 +601,8 @@ __global__ void __launch_bounds__(THREADS) k_pauli_pair(V<R>* __restrict__ a, ui
 }
 
 // The kernels of a measurement may launch under the end of the kernel before them (launch_measure):
-// they touch nothing before that one is done.  Each takes 2 to 5 us at 17 qubits and waited as long for its
+// they touch nothing before that one is done, and read the register through plain pointers (const and
+// __restrict__ would promise memory that nobody writes while they are resident).  Each takes 2 to 5 us at 17 qubits and waited as long for its
 // launch: a noisy trajectory with 48 measurements 1050 -> 888 us; n = 6 710 -> 583, n = 20 1633 -> 1467,
 // n = 22 and above within 3% (faster).
 __device__ __forceinline__ void after_previous_kernel() {
@@ -783,7 +784,7 @@ __device__ void decide_in_last_block(const double* partials, MeasureQueue* q, in
 
 // <psi|P|psi> (and optionally <psi|psi>): slots re, im[, norm]; with a queue the measurement's outcome too
 template <class R, bool NORM>
-__global__ void __launch_bounds__(REDUCE_THREADS) k_expect_diag(const V<R>* __restrict__ a, uint64_t len, uint64_t z, int ph,
+__global__ void __launch_bounds__(REDUCE_THREADS) k_expect_diag(const V<R>* a, uint64_t len, uint64_t z, int ph,
                                                                 double* partials, MeasureQueue* queue = nullptr, int slot = 0) {
   after_previous_kernel();
   // sum_c i^{k(c)} |psi(c)|^2
@@ -809,7 +810,7 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_expect_diag(const V<R>* __re
 }
 
 template <class R, bool NORM>
-__global__ void __launch_bounds__(REDUCE_THREADS) k_expect_pair(const V<R>* __restrict__ a, uint64_t npairs, int h, uint64_t x,
+__global__ void __launch_bounds__(REDUCE_THREADS) k_expect_pair(const V<R>* a, uint64_t npairs, int h, uint64_t x,
                                                                 uint64_t z, int ph, double* partials,
                                                                 MeasureQueue* queue = nullptr, int slot = 0) {
   after_previous_kernel();
@@ -1601,7 +1602,6 @@ int launch_project_partials(ncsim_state* s, uint64_t x, uint64_t z, uint32_t pha
 
 bool can_measure_on_device(const ncsim_state* s) { return reduce_grid(s->len) <= DECIDE_BLOCKS; }
 
-// measurement `slot` of the queue: outcome and projection, nothing waited for; a reset also flips on 1
 // a kernel that calls after_previous_kernel first, launched under the end of the stream's last kernel
 template <class... P, class... A>
 static void launch_under(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t stream, A... args) {
@@ -1617,6 +1617,7 @@ static void launch_under(void (*kernel)(P...), unsigned grid, unsigned block, cu
   NCSIM_CUDA(cudaLaunchKernelEx(&launch, kernel, P(args)...));
 }
 
+// measurement `slot` of the queue: outcome and projection, nothing waited for; a reset also flips on 1
 void launch_measure(ncsim_state* s, uint64_t x, uint64_t z, uint32_t phase, MeasureQueue* queue, int slot, bool reset) {
   const int ph = int(phase & 3);
   const int* decided = &queue->outcome[slot];
