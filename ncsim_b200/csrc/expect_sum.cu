@@ -313,38 +313,35 @@ void state_expectations(const ncsim_state* s, uint64_t count, const uint64_t* x,
     passes.push_back(std::move(p));
     left.swap(rest);
   }
-  uint32_t total = 0;
-  for (const auto& p : passes) total += p.terms;
-  const unsigned blocks = unsigned(std::min<uint64_t>(s->len >> T, uint64_t(sm_count()) * 2));
-  double *partials = nullptr, *d_out = nullptr;
-  NCSIM_CUDA(pool_alloc(&partials, size_t(ES_TERMS) * blocks * sizeof(double), s->stream));
-  NCSIM_CUDA(pool_alloc(&d_out, total * sizeof(double), s->stream));
-  uint32_t at = 0;
-  for (const auto& p : passes) {
-    if (s->precision == NCSIM_C128) launch_pass<double>(s, p, z, partials, d_out + at, blocks);
-    else launch_pass<float>(s, p, z, partials, d_out + at, blocks);
-    at += p.terms;
-  }
-  std::vector<double> v(total);
-  NCSIM_CUDA(cudaMemcpyAsync(v.data(), d_out, total * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-  NCSIM_CUDA(cudaFreeAsync(partials, s->stream));
-  NCSIM_CUDA(cudaFreeAsync(d_out, s->stream));
-  NCSIM_CUDA(cudaStreamSynchronize(s->stream));
-  at = 0;
-  for (const auto& p : passes)
-    for (const auto& g : p.groups)
-      for (uint32_t k : g.second) {
-        const double a = v[at++];
-        // i^phase times the sum: 2 Re s, 2 i Im s, or the diagonal's
-        const uint32_t odd = uint32_t(__builtin_popcountll(z[k] & g.first) & 1);
-        const double m = g.first ? 2.0 * a : a;
-        switch ((phase[k] + odd) & 3u) {
-          case 0: out[k] = {m, 0.0}; break;
-          case 1: out[k] = {0.0, m}; break;
-          case 2: out[k] = {-m, 0.0}; break;
-          default: out[k] = {0.0, -m}; break;
+  // Scratch is the state's own, as for a single Pauli: block partials in its reduction scratch (one pass
+  // after another), the sums written by the device to its pinned mirror, waited for when that is full.
+  constexpr size_t SLOTS = size_t(MAX_REDUCE_BLOCKS) * PARTIAL_SLOTS;
+  const unsigned blocks =
+      unsigned(std::min<uint64_t>({s->len >> T, uint64_t(sm_count()) * 2, uint64_t(SLOTS / ES_TERMS)}));
+  for (size_t first = 0; first < passes.size();) {
+    size_t end = first, at = 0;
+    for (; end < passes.size() && at + passes[end].terms <= SLOTS; ++end) {
+      if (s->precision == NCSIM_C128) launch_pass<double>(s, passes[end], z, s->partials, s->host_partials + at, blocks);
+      else launch_pass<float>(s, passes[end], z, s->partials, s->host_partials + at, blocks);
+      at += passes[end].terms;
+    }
+    NCSIM_CUDA(cudaStreamSynchronize(s->stream));
+    const double* v = s->host_partials;
+    for (; first < end; ++first)
+      for (const auto& g : passes[first].groups)
+        for (uint32_t k : g.second) {
+          const double a = *v++;
+          // i^phase times the sum: 2 Re s, 2 i Im s, or the diagonal's
+          const uint32_t odd = uint32_t(__builtin_popcountll(z[k] & g.first) & 1);
+          const double m = g.first ? 2.0 * a : a;
+          switch ((phase[k] + odd) & 3u) {
+            case 0: out[k] = {m, 0.0}; break;
+            case 1: out[k] = {0.0, m}; break;
+            case 2: out[k] = {-m, 0.0}; break;
+            default: out[k] = {0.0, -m}; break;
+          }
         }
-      }
+  }
 }
 
 }  // namespace ncsim
