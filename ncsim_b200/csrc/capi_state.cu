@@ -165,7 +165,8 @@ ncsim_state* state_new(uint32_t n, int32_t precision) {
     NCSIM_CUDA(cudaGetDevice(&s->device));
     NCSIM_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     NCSIM_CUDA(cudaMalloc(&s->amp, s->bytes()));
-    NCSIM_CUDA(cudaMalloc(&s->partials, sizeof(double) * MAX_REDUCE_BLOCKS * PARTIAL_SLOTS));
+    NCSIM_CUDA(cudaMalloc(&s->partials, sizeof(double) * MAX_REDUCE_BLOCKS * PARTIAL_SLOTS + sizeof(MeasureQueue)));
+    s->queue = reinterpret_cast<MeasureQueue*>(s->partials + MAX_REDUCE_BLOCKS * PARTIAL_SLOTS);
     NCSIM_CUDA(cudaMallocHost(&s->host_partials, sizeof(double) * MAX_REDUCE_BLOCKS * PARTIAL_SLOTS));
     NCSIM_CUDA(cudaMalloc(&s->dev_flag, 256));
   } catch (...) {

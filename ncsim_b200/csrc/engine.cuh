@@ -98,6 +98,16 @@ constexpr int REDUCE_THREADS = 512;
 constexpr int MAX_REDUCE_BLOCKS = 4096;
 constexpr int PARTIAL_SLOTS = 4;  // doubles per block partial
 
+// Measurements of a run decided on the device: the uniforms that they may need, drawn ahead in stream order
+// (an uncertain outcome takes the next one), and the outcomes.
+constexpr int MEASURE_QUEUE = 256;
+struct MeasureQueue {
+  double uniform[MEASURE_QUEUE];
+  int outcome[MEASURE_QUEUE];
+  uint32_t used;    // uniforms taken
+  uint32_t ticket;  // blocks of the current reduction that have stored their partial
+};
+
 }  // namespace ncsim
 
 namespace ncsim {
@@ -122,7 +132,8 @@ struct ncsim_state {
   void* amp = nullptr;      // device: double2[len] or float2[len]
   cudaStream_t stream = nullptr;
   int device = 0;
-  double* partials = nullptr;       // device scratch: MAX_REDUCE_BLOCKS * PARTIAL_SLOTS
+  double* partials = nullptr;       // device scratch: MAX_REDUCE_BLOCKS * PARTIAL_SLOTS, then `queue`
+  ncsim::MeasureQueue* queue = nullptr;  // device: the measurements of a run (in the partials' allocation)
   double* host_partials = nullptr;  // pinned mirror of `partials`
   int* dev_flag = nullptr;          // device word: a pass kernel's error code (kept for the state's life)
   mutable std::recursive_mutex mu;
@@ -313,15 +324,6 @@ int launch_project_partials(ncsim_state* s, uint64_t x, uint64_t z, uint32_t pha
 // slots: <a|b> re, im, <a|a>, <b|b>; the per-block max |a-b| goes to maxdiff_dev[block]
 int launch_compare_partials(const ncsim_state* a, const ncsim_state* b, double* maxdiff_dev);
 // sampling
-// Measurements of a run decided on the device: the uniforms that they may need, drawn ahead in stream order
-// (an uncertain outcome takes the next one), and the outcomes.
-constexpr int MEASURE_QUEUE = 256;
-struct MeasureQueue {
-  double uniform[MEASURE_QUEUE];
-  int outcome[MEASURE_QUEUE];
-  uint32_t used;    // uniforms taken
-  uint32_t ticket;  // blocks of the current reduction that have stored their partial
-};
 bool can_measure_on_device(const ncsim_state* s);
 void launch_measure(ncsim_state* s, uint64_t x, uint64_t z, uint32_t phase, MeasureQueue* queue, int slot, bool reset);
 void launch_block_weights(const ncsim_state* s, double* weights_dev, uint64_t nblocks, uint64_t block);

@@ -457,9 +457,6 @@ class QueuedMeasurements {
  public:
   QueuedMeasurements(ncsim_state* s, const ncsim_circuit* c, ncsim_rng* rng, uint8_t* rec, size_t* m)
       : s_(s), c_(c), rng_(rng), rec_(rec), m_(m) {}
-  ~QueuedMeasurements() {
-    if (dev_) cudaFreeAsync(dev_, s_->stream);
-  }
   // op i of the circuit, a measurement or a reset of a Hermitian Pauli
   void add(size_t i) {
     if (count_ == MEASURE_QUEUE) flush();
@@ -467,7 +464,7 @@ class QueuedMeasurements {
     const OpIR& op = c_->ops[i];
     const bool reset = op.kind == OpKind::Reset;
     const uint64_t x = reset ? 0 : op.pauli.x, z = reset ? uint64_t(1) << op.qubits[0] : op.pauli.z;
-    launch_measure(s_, x, z, reset ? 0 : op.pauli.phase, dev_, int(count_), reset);
+    launch_measure(s_, x, z, reset ? 0 : op.pauli.phase, s_->queue, int(count_), reset);
     recorded_[count_++] = !reset;
   }
   void flush() {
@@ -478,7 +475,7 @@ class QueuedMeasurements {
     };
     static_assert(offsetof(MeasureQueue, used) == offsetof(MeasureQueue, outcome) + offsetof(Back, used), "one copy");
     auto* back = reinterpret_cast<Back*>(s_->host_partials);  // pinned
-    NCSIM_CUDA(cudaMemcpyAsync(back, dev_->outcome, sizeof(Back), cudaMemcpyDeviceToHost, s_->stream));
+    NCSIM_CUDA(cudaMemcpyAsync(back, s_->queue->outcome, sizeof(Back), cudaMemcpyDeviceToHost, s_->stream));
     NCSIM_CUDA(cudaStreamSynchronize(s_->stream));
     for (uint32_t k = 0; k < back->used; ++k) rng_->f64();
     for (size_t k = 0; k < count_; ++k)
@@ -488,20 +485,18 @@ class QueuedMeasurements {
 
  private:
   void begin(size_t i) {
-    if (!dev_) NCSIM_CUDA(pool_alloc(&dev_, sizeof(MeasureQueue), s_->stream));
     MeasureQueue q{};
     ncsim_rng ahead = *rng_;
     int k = 0;  // at most one draw per measurement up to the next op that draws by itself
     for (size_t j = i; j < c_->ops.size() && k < MEASURE_QUEUE && c_->ops[j].kind != OpKind::Noise; ++j)
       if (c_->ops[j].kind == OpKind::Measure || c_->ops[j].kind == OpKind::Reset) q.uniform[k++] = ahead.f64();
-    NCSIM_CUDA(cudaMemcpyAsync(dev_, &q, sizeof(q), cudaMemcpyHostToDevice, s_->stream));
+    NCSIM_CUDA(cudaMemcpyAsync(s_->queue, &q, sizeof(q), cudaMemcpyHostToDevice, s_->stream));
   }
   ncsim_state* s_;
   const ncsim_circuit* c_;
   ncsim_rng* rng_;
   uint8_t* rec_;
   size_t* m_;
-  MeasureQueue* dev_ = nullptr;
   size_t count_ = 0;
   bool recorded_[MEASURE_QUEUE];
 };

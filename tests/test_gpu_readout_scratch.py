@@ -22,3 +22,15 @@ def test_expectation_sum_takes_nothing_from_the_pool():
     assert nb.pool_info() == before
     # <+|P|+> is 1 without Z and 0 with it
     assert abs(got - ((1 << 10) + 0.5 * 14 * (1 << 10))) < 1e-9
+
+
+@pytest.mark.parametrize("n", [1, 12])
+def test_measurements_of_a_run_take_nothing_from_the_pool(n):
+    import ncsim_b200 as nb
+
+    c = nb.Circuit.parse(f"QUBITS {n}\nH 0\nM 0\nR 0\nH 0\nMPP X0\n")
+    s, rng = nb.GpuStateVector(n), nb.StdRng(1)
+    nb.trim_memory()
+    before = nb.pool_info()
+    assert s.run(c, rng)[1] is False  # |+> measured in X
+    assert nb.pool_info() == before
