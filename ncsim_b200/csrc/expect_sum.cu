@@ -313,18 +313,21 @@ void state_expectations(const ncsim_state* s, uint64_t count, const uint64_t* x,
     passes.push_back(std::move(p));
     left.swap(rest);
   }
-  // Scratch is the state's own, as for a single Pauli: block partials in its reduction scratch (one pass
-  // after another), the sums written by the device to its pinned mirror, waited for when that is full.
+  // Scratch is the state's own, as for a single Pauli: in its reduction scratch the block partials (one
+  // pass after another) and behind them the sums, fetched when the room is used up.
   constexpr size_t SLOTS = size_t(MAX_REDUCE_BLOCKS) * PARTIAL_SLOTS;
   const unsigned blocks =
-      unsigned(std::min<uint64_t>({s->len >> T, uint64_t(sm_count()) * 2, uint64_t(SLOTS / ES_TERMS)}));
+      unsigned(std::min<uint64_t>({s->len >> T, uint64_t(sm_count()) * 2, uint64_t(SLOTS / ES_TERMS - 1)}));
+  double* const sums = s->partials + size_t(ES_TERMS) * blocks;
+  const size_t room = SLOTS - size_t(ES_TERMS) * blocks;
   for (size_t first = 0; first < passes.size();) {
     size_t end = first, at = 0;
-    for (; end < passes.size() && at + passes[end].terms <= SLOTS; ++end) {
-      if (s->precision == NCSIM_C128) launch_pass<double>(s, passes[end], z, s->partials, s->host_partials + at, blocks);
-      else launch_pass<float>(s, passes[end], z, s->partials, s->host_partials + at, blocks);
+    for (; end < passes.size() && at + passes[end].terms <= room; ++end) {
+      if (s->precision == NCSIM_C128) launch_pass<double>(s, passes[end], z, s->partials, sums + at, blocks);
+      else launch_pass<float>(s, passes[end], z, s->partials, sums + at, blocks);
       at += passes[end].terms;
     }
+    NCSIM_CUDA(cudaMemcpyAsync(s->host_partials, sums, at * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     NCSIM_CUDA(cudaStreamSynchronize(s->stream));
     const double* v = s->host_partials;
     for (; first < end; ++first)
