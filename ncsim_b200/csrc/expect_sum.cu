@@ -268,11 +268,25 @@ void launch_pass(const ncsim_state* s, const EsPass& pass, const uint64_t* z, do
 
 }  // namespace
 
+// The fewest terms that a pass is made for; fewer go one Pauli at a time.  While the register
+// stays in the L2 the wait for a single Pauli outweighs a pass (8 terms in windows of their own,
+// n = 20: 178 us one by one, 139 in passes; n = 22 238 and 207).  From 128 MiB on one Pauli streams the
+// register faster than a pass (the same terms, n = 23: 338 and 387, n = 28 4.9 and 10.0 ms), two
+// do not (n = 26 1.41 and 1.26 ms), unless a window of scattered qubits reads a complex128 register
+// of some GiB in short runs (n = 30 19.3 and 22.8 ms; three terms 22.2 and 15.2; a window of low qubits
+// 5.2 and 4.7; complex64 16.2 and 13.6).
+uint32_t least_terms(const ncsim_state* s, uint64_t window) {
+  if (s->bytes() < (size_t(128) << 20)) return 1;
+  const bool short_runs = (window & 127) != 127;
+  return s->precision == NCSIM_C128 && s->bytes() >= (size_t(4) << 30) && short_runs ? 3 : 2;
+}
+
 CplxD state_expectation(const ncsim_state* s, uint64_t x, uint64_t z, uint32_t phase);
 void check_pauli_on(const ncsim_state* s, uint64_t x, uint64_t z);
 
 // <psi|P_k|psi> of every term.  Terms whose X part spans more qubits than a window holds, and
-// registers of fewer than 8 qubits, go one Pauli at a time; so does a single term.
+// registers of fewer than 8 qubits, go one Pauli at a time; so does a single term, and so do the
+// terms of a pass that would have too few (least_terms).
 void state_expectations(const ncsim_state* s, uint64_t count, const uint64_t* x, const uint64_t* z, const uint32_t* phase,
                         CplxD* out) {
   for (uint64_t k = 0; k < count; ++k) check_pauli_on(s, x[k], z[k]);
@@ -310,8 +324,13 @@ void state_expectations(const ncsim_state* s, uint64_t count, const uint64_t* x,
       if (n < g.second.size()) rest.push_back({g.first, std::vector<uint32_t>(g.second.begin() + long(n), g.second.end())});
     }
     for (int q = 0; __builtin_popcountll(p.window) < T; ++q) p.window |= uint64_t(1) << q;
-    passes.push_back(std::move(p));
     left.swap(rest);
+    if (p.terms >= least_terms(s, p.window)) {
+      passes.push_back(std::move(p));
+      continue;
+    }
+    for (const auto& g : p.groups)
+      for (uint32_t k : g.second) out[k] = state_expectation(s, x[k], z[k], phase[k] & 3);
   }
   // Scratch is the state's own, as for a single Pauli: in its reduction scratch the block partials (one
   // pass after another) and behind them the sums, fetched when the room is used up.
