@@ -104,9 +104,11 @@ enum DevKind : uint32_t {
   DK_RZ_OUT = DK_RZ + CUBE_BITS,     // two phases selected by a tile bit outside the cube
   DK_SWAP,                           // + index of the xor mask: exchange inside the cube (no phases)
   DK_SWAPC = DK_SWAP + 10,           // + index of the xor mask: exchange with phases
-  DK_TABLE = DK_SWAPC + 10,          // phase table
+  DK_POLY_CONST = DK_SWAPC + 10,     // phase polynomial without terms: the same phase on every element
+  // outside the chains, sweeps over the tile:
+  DK_TABLE,                          // phase table
   DK_POLY,                           // phase polynomial
-  DK_TILE_SWAP,                      // exchange across more than two tile bits: its own sweep over the tile
+  DK_TILE_SWAP,                      // exchange across more than two tile bits
   DK_COND = 0x8000,                  // set when the op has fixed bits outside the window (gfix, gval)
 };
 // the xor masks of an exchange on one or two cube bits, in DK_SWAP's order
@@ -150,7 +152,7 @@ template <class R>
 struct alignas(16) OpArgs {
   union {
     V<R> c[4];
-    uint32_t a[8];    // table: k, lfix, lones, up, cp; polynomial: k, up, cp, parity offset; tile swap: see tile_pairswap;
+    uint32_t a[8];    // table: k, up, cp, lfix, lones; polynomial: k, up, cp, parity offset; tile swap: see tile_pairswap;
   };                  // chain: the tile bits of the thread's index, one byte each, in a[0], a[1]
 };
 struct DevOp {
@@ -178,15 +180,6 @@ __host__ __device__ __forceinline__ uint64_t tile_base_of(uint64_t t, const Pass
   for (int i = 0; i < g.nh; ++i) {
     const int b = g.hq[i];
     v = ((v >> b) << (b + 1)) | (v & ((uint64_t(1) << b) - 1));
-  }
-  return v;
-}
-
-// v with zero bits inserted at the ascending local positions pos[0..cnt)
-__device__ __forceinline__ uint32_t insert_zeros32(uint32_t v, const uint8_t* pos, int cnt) {
-  for (int i = 0; i < cnt; ++i) {
-    const int b = pos[i];
-    v = ((v >> b) << (b + 1)) | (v & ((1u << b) - 1));
   }
   return v;
 }
@@ -234,20 +227,39 @@ __device__ __forceinline__ double flip(double x, uint32_t s) {
 }
 __device__ __forceinline__ float flip(float x, uint32_t s) { return __uint_as_float(__float_as_uint(x) ^ s); }
 
-// exchange across three or more tile bits: a: number of fixed bits, their positions in the word pool, pairswap flags, xor mask, values
+// exchange across three or more tile bits: a: number of fixed bits, pairswap flags, xor mask, values, constants,
+// and the fixed bits' positions, four bits each, in a[6], a[7]
 template <class R>
-__device__ void tile_pairswap(SwTile<R> t, uint32_t tsz, const OpArgs<R>& op, const V<R>* cpool, const uint32_t* up) {
-  const int nf = int(op.a[0]);
-  uint8_t pos[MAX_TILE_BITS];
-  for (int i = 0; i < nf; ++i) pos[i] = uint8_t(up[op.a[1] + i]);
-  const bool ui = op.a[2] & 1, uj = (op.a[2] >> 1) & 1;
-  const V<R> ci = cpool[op.a[5]], cj = cpool[op.a[5] + 1];
-  for (uint32_t p = threadIdx.x; p < (tsz >> nf); p += blockDim.x) {
-    const uint32_t i = insert_zeros32(p, pos, nf) | op.a[4];
-    const uint32_t j = i ^ op.a[3];
-    const V<R> vi = t[i], vj = t[j];
-    t[i] = ui ? vj : cmul(ci, vj);
-    t[j] = uj ? vi : cmul(cj, vi);
+__device__ __forceinline__ void tile_pairswap(SwTile<R> t, uint32_t tsz, const OpArgs<R>& op, const V<R>* cpool) {
+  const uint32_t nf = op.a[0], pairs = tsz >> nf, x = op.a[2], ones = op.a[3];
+  const uint64_t fixed = uint64_t(op.a[7]) << 32 | op.a[6];
+  const bool ui = op.a[1] & 1, uj = (op.a[1] >> 1) & 1;
+  V<R> ci{}, cj{};
+  if (!(ui && uj)) ci = cpool[op.a[4]], cj = cpool[op.a[4] + 1];
+  constexpr int N = 8;  // pairs in flight: a thread has eight of a tile's at most
+  for (uint32_t p = threadIdx.x; p < pairs; p += N * blockDim.x) {
+    uint32_t i[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u) i[u] = p + u * blockDim.x < pairs ? p + u * blockDim.x : p;  // its own pair again
+    uint64_t pos = fixed;
+    for (uint32_t f = 0; f < nf; ++f, pos >>= 4) {
+      const uint32_t b = uint32_t(pos) & 15u, low = (1u << b) - 1;
+#pragma unroll
+      for (int u = 0; u < N; ++u) i[u] = ((i[u] & ~low) << 1) | (i[u] & low);
+    }
+    V<R> vi[N], vj[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      i[u] |= ones;
+      vi[u] = t[i[u]];
+      vj[u] = t[i[u] ^ x];
+    }
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+      if (p + u * blockDim.x < pairs) {
+        t[i[u]] = ui ? vj[u] : cmul(ci, vj[u]);
+        t[i[u] ^ x] = uj ? vi[u] : cmul(cj, vi[u]);
+      }
   }
 }
 
@@ -442,6 +454,28 @@ __device__ __forceinline__ void chain_flush(V<R> (&v)[CUBE], uint32_t& pend) {
   pend = 0;
 }
 
+// v times the phase of the polynomial's value f (u: the polynomial's words)
+template <class R>
+__device__ __forceinline__ V<R> phase_of_value(V<R> v, uint32_t f, const uint32_t* u, const V<R>* cp) {
+  if (is_zero(v)) return v;
+  const uint32_t bits = u[0];
+  const bool use_table = u[1], s_one = u[2];
+  if (bits < 32) f &= (1u << bits) - 1;
+  V<R> c;
+  if (use_table) {
+    c = cp[1 + f];
+    if (is_one_v(c)) return v;
+  } else {
+    if (f == 0 && s_one) return v;
+    const double2 rr = pass_root(f, bits);
+    c.x = R(rr.x);
+    c.y = R(rr.y);
+    if (!s_one) c = cmul(cp[0], c);
+  }
+  return cmul(c, v);
+}
+
+// v times the phase of a polynomial at index i
 template <class R>
 __device__ __forceinline__ V<R> phasepoly_elem(V<R> v, uint64_t i, const OpArgs<R>& op, const PassParams<R>& P) {
   if (is_zero(v)) return v;
@@ -475,16 +509,80 @@ __device__ __forceinline__ V<R> phasepoly_elem(V<R> v, uint64_t i, const OpArgs<
   return cmul(c, v);
 }
 
+// The ops outside the chains, one at a time over the tile (element round r of a thread: threadIdx.x + r * blockDim.x).
+// Patterns and parities are linear in the index: the thread's part is made once and each round adds its own.
+// Evaluated in the chains, element by element with a loop over their qubits or parities, they held up 16 elements at
+// once: 30 tables on 8 qubits at n = 10 209 us, here 92 (in chains of 8 elements to each of 512 threads 115), at n = 28
+// 53 ms, 28 (47); 30 polynomials of two terms with H between at n = 28 192 ms, 56 (138).  Exchanges across five bits,
+// 40 of them at n = 10: 81 us one pair at a time, 61 with all eight in flight.  Not inlined: the op loop keeps its registers.
 template <class R>
-__device__ __forceinline__ V<R> table_elem(V<R> v, uint32_t e, uint32_t xout, const OpArgs<R>& op, const PassParams<R>& P) {
-  const int k = int(op.a[0]);
-  if ((e & op.a[1]) != op.a[2]) return v;
-  const uint32_t* qp = P.upool + op.a[3];
-  const uint8_t* unit = reinterpret_cast<const uint8_t*>(qp + k);
-  uint32_t x = xout;
-  for (int j = 0; j < k; ++j)
-    if (qp[j] < 256) x |= ((e >> qp[j]) & 1u) << j;
-  return unit[x] ? v : cmul(P.cpool[op.a[4] + x], v);
+__device__ __noinline__ void tile_sweep(uint32_t kind, uint32_t buf, uint64_t base, uint64_t dthread, const uint64_t* dround,
+                                        const OpArgs<R>& op, const PassParams<R>& P) {
+  const SwTile<R> t{shared_tile<R>() + buf};
+  const uint32_t tsz = 1u << P.g.T;
+  const uint32_t nr = (tsz + blockDim.x - 1) / blockDim.x, lb = 31u - __clz(blockDim.x);  // a round moves tile bits lb and up
+  if (kind == DK_TILE_SWAP) {
+    tile_pairswap<R>(t, tsz, op, P.cpool);
+  } else if (kind == DK_TABLE) {
+    const uint32_t k = op.a[0], lfix = op.a[3], lones = op.a[4];
+    const uint32_t* qp = P.upool + op.a[1];
+    const uint8_t* unit = reinterpret_cast<const uint8_t*>(qp + k);
+    const V<R>* c = P.cpool + op.a[2];
+    uint32_t x0 = 0, w[CUBE_BITS] = {};
+    for (uint32_t j = 0; j < k; ++j) {
+      const uint32_t q = qp[j];
+      x0 |= (q >= 256 ? uint32_t(base >> (q - 256)) & 1u : (threadIdx.x >> q) & 1u) << j;
+#pragma unroll
+      for (int i = 0; i < CUBE_BITS; ++i) w[i] |= uint32_t(q == lb + i) << j;
+    }
+    for (uint32_t r0 = 0; r0 < nr; r0 += 4) {  // four elements in flight
+      V<R> u[4], f[4];
+      uint32_t leave[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t r = r0 + i, e = threadIdx.x + r * blockDim.x;
+        uint32_t x = x0;
+#pragma unroll
+        for (int j = 0; j < CUBE_BITS; ++j) x |= ((r >> j) & 1) ? w[j] : 0u;
+        u[i] = t[e];
+        f[i] = c[x];
+        leave[i] = unit[x] | uint32_t((e & lfix) != lones);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (!leave[i]) t[threadIdx.x + (r0 + i) * blockDim.x] = cmul(f[i], u[i]);
+    }
+  } else {  // DK_POLY
+    const uint32_t* u = P.upool + op.a[1];
+    const uint64_t* pp = P.ppool + op.a[3];
+    const uint32_t nt = op.a[0];
+    const uint32_t* start = u + 5;
+    const uint32_t* coeff = start + nt + 1;
+    const uint64_t i = base | dthread;
+    // a parity is one mask over the rounds, a term's rounds are the AND of its parities' masks
+    uint32_t in[MAX_PASS_TERMS] = {}, co[MAX_PASS_TERMS] = {};
+#pragma unroll
+    for (uint32_t k = 0; k < MAX_PASS_TERMS; ++k)
+      if (k < nt) {
+        uint32_t m = 0xffffu;
+        for (uint32_t l = start[k]; l < start[k + 1]; ++l) {
+          const uint64_t p = pp[l];
+          const auto odd = [&](uint64_t x) { return __popcll(p & x) & 1; };
+          m &= (odd(i) ? 0xffffu : 0u) ^ (odd(dround[1]) ? 0xaaaau : 0u) ^ (odd(dround[2]) ? 0xccccu : 0u) ^
+               (odd(dround[4]) ? 0xf0f0u : 0u) ^ (nr > 8 && odd(dround[8]) ? 0xff00u : 0u);
+        }
+        in[k] = m;
+        co[k] = coeff[k];
+      }
+    const uint32_t constant = u[3];  // a value has at most 32 bits
+    for (uint32_t r = 0; r < nr; ++r) {
+      uint32_t f = constant;
+#pragma unroll
+      for (uint32_t k = 0; k < MAX_PASS_TERMS; ++k) f += ((in[k] >> r) & 1u) ? co[k] : 0u;
+      V<R>& at = t[threadIdx.x + r * blockDim.x];
+      at = phase_of_value<R>(at, f, u, P.cpool + op.a[2]);
+    }
+  }
 }
 
 // The chain whose head is op o.  gbase: the tile bits of the thread's cube (its index
@@ -581,23 +679,10 @@ __device__ __forceinline__ void tile_chain(uint32_t tile, uint32_t o, uint32_t g
       }
       case DK_FLUSH: chain_flush<R>(v, pend); break;
       case DK_RZ_OUT: chain_phase<R, -1>(v, op.c[on ? 1 : 0]); break;
-      case DK_TABLE: {
-        const int k = int(op.a[0]);
-        const uint32_t* qp = P.upool + op.a[3];
-        uint32_t xout = 0;
-        for (int j = 0; j < k; ++j)
-          if (qp[j] >= 256) xout |= uint32_t((base >> (qp[j] - 256)) & 1u) << j;
-#pragma unroll
-        for (int b = 0; b < CUBE; ++b) {
-          uint32_t e = gb;
-#pragma unroll
-          for (int j = 0; j < CUBE_BITS; ++j)
-            if ((b >> j) & 1) e |= lb[j];
-          v[b] = table_elem<R>(v[b], e, xout, op, P);
-        }
-        break;
-      }
-      case DK_POLY: {
+      case DK_POLY_CONST: {
+        // Polynomials with terms are sweeps.  The general form stands here because the compiler lays out the whole
+        // switch by it: without this case, or with a short one, it copies a complex128 cube's registers at every op
+        // (random layers at n = 28 91 -> 148 and 103 ms).
 #pragma unroll
         for (int b = 0; b < CUBE; ++b) {
           uint32_t e = gb;
@@ -696,9 +781,9 @@ __global__ void __launch_bounds__(3 * PASS_THREADS) k_plain_pass(const __grid_co
       if (h.kind == DK_CHAIN) {
         tile_chain<R>(buf, o, cubes[h.gvl * blockDim.x + threadIdx.x], args, signs, P, base);
         o += h.em;
-      } else {  // DK_TILE_SWAP
+      } else {
         if ((base & P.cond[o].gfix) != P.cond[o].gval) continue;
-        tile_pairswap<R>(SwTile<R>{shared_tile<R>() + buf}, tsz, args[o], P.cpool, P.upool);
+        tile_sweep<R>(h.kind & ~uint32_t(DK_COND), buf, base, dthread, dround, args[o], P);
       }
       __syncthreads();
     }
@@ -1041,8 +1126,12 @@ uint32_t coupled_bits(const TileOp& op) {
   }
 }
 
-// the exchange of a chain spans one or two cube bits; wider ones sweep the tile by themselves
-bool chainable(const TileOp& op) { return op.kind != TK_PAIRSWAP || __builtin_popcount(op.lx) <= 2; }
+// whether an op goes into a chain: tables, polynomials and exchanges across more than two bits sweep the tile by themselves
+bool chainable(const TileOp& op) {
+  if (op.kind == TK_DIAG_TABLE) return false;
+  if (op.kind == TK_PHASEPOLY) return op.k == 0;
+  return op.kind != TK_PAIRSWAP || __builtin_popcount(op.lx) <= 2;
+}
 
 // Orders a chain's thread bits: the lowest SB (a quarter warp of 16-byte elements, half a
 // warp of 8-byte ones) on tile bits of distinct residues mod SB, so that their accesses
@@ -1074,17 +1163,31 @@ std::vector<DevOp> chainify(const std::vector<TileOp>& ops, int T, PlainPlan& P,
     if (!chainable(ops[i])) {
       const TileOp& op = ops[i++];
       DevOp d{};
-      d.h.kind = DK_TILE_SWAP;
       d.g.gfix = op.gfix;
       d.g.gval = op.gval;
-      d.x.a[0] = uint32_t(__builtin_popcount(op.lfix));
-      d.x.a[1] = uint32_t(P.upool.size());
-      for (int b = 0; b < T; ++b)
-        if ((op.lfix >> b) & 1) P.upool.push_back(uint32_t(b));
-      d.x.a[2] = op.flags;
-      d.x.a[3] = op.lx;
-      d.x.a[4] = op.lones;
-      d.x.a[5] = op.cp;
+      if (op.kind == TK_DIAG_TABLE) {
+        d.h.kind = DK_TABLE;
+        d.x.a[0] = op.k;
+        d.x.a[1] = op.up;
+        d.x.a[2] = op.cp;
+        d.x.a[3] = op.lfix;
+        d.x.a[4] = op.lones;
+      } else if (op.kind == TK_PHASEPOLY) {
+        d.h.kind = DK_POLY;
+        d.x.a[0] = op.k;
+        d.x.a[1] = op.up;
+        d.x.a[2] = op.cp;
+        d.x.a[3] = uint32_t(op.gz);
+      } else {
+        d.h.kind = DK_TILE_SWAP;
+        d.x.a[0] = uint32_t(__builtin_popcount(op.lfix));
+        d.x.a[1] = op.flags;
+        d.x.a[2] = op.lx;
+        d.x.a[3] = op.lones;
+        d.x.a[4] = op.cp;
+        for (int b = 0, f = 0; b < T; ++b)
+          if ((op.lfix >> b) & 1) d.x.a[6 + f / 8] |= uint32_t(b) << (4 * (f & 7)), ++f;
+      }
       out.push_back(d);
       continue;
     }
@@ -1229,17 +1332,8 @@ std::vector<DevOp> chainify(const std::vector<TileOp>& ops, int T, PlainPlan& P,
           }
           break;
         }
-        case TK_DIAG_TABLE:
-          d.h.kind = DK_TABLE;
-          d.h.gml = d.h.gvl = 0;  // the fixed bits are compared per element
-          d.x.a[0] = op.k;
-          d.x.a[1] = op.lfix;
-          d.x.a[2] = op.lones;
-          d.x.a[3] = op.up;
-          d.x.a[4] = op.cp;
-          break;
         default:  // TK_PHASEPOLY
-          d.h.kind = DK_POLY;
+          d.h.kind = DK_POLY_CONST;
           d.h.gml = d.h.gvl = 0;
           d.x.a[0] = op.k;
           d.x.a[1] = op.up;
@@ -1260,7 +1354,7 @@ std::vector<DevOp> chainify(const std::vector<TileOp>& ops, int T, PlainPlan& P,
 // whether an op of this kind carries constants (else words)
 bool has_constants(uint32_t kind) {
   kind &= ~uint32_t(DK_COND);
-  return (kind >= DK_D1 && kind <= DK_PH_MASK) || (kind >= DK_RZ && kind <= DK_RZ_OUT) || (kind >= DK_SWAPC && kind < DK_TABLE);
+  return (kind >= DK_D1 && kind <= DK_PH_MASK) || (kind >= DK_RZ && kind <= DK_RZ_OUT) || (kind >= DK_SWAPC && kind < DK_POLY_CONST);
 }
 void put_args(OpArgs<double>& to, const DevOp& from) { to = from.x; }
 void put_args(OpArgs<float>& to, const DevOp& from) {
