@@ -296,6 +296,7 @@ __device__ __forceinline__ double2 pass_root(uint64_t f, uint32_t bits) {
 // bits on finite amplitudes more cheaply is used: products with exact zeros are
 // left out (real matrices), +-i exchanges the parts, and -1 is a sign flip, which
 // commutes with every rounding and so waits in a mask until an op mixes elements.
+// (Tiles with other amplitudes are done over with every product: redo_tile.)
 // The updates are written so that each result can take the place of an operand
 // that has just been read for the last time (both products with a0 first): the
 // cases of the op loop then meet on the same registers without copies between.
@@ -586,10 +587,11 @@ __device__ __noinline__ void tile_sweep(uint32_t kind, uint32_t buf, uint64_t ba
 }
 
 // The chain whose head is op o.  gbase: the tile bits of the thread's cube (its index
-// spread over the tile bits outside the cube).
-template <class R>
-__device__ __forceinline__ void tile_chain(uint32_t tile, uint32_t o, uint32_t gbase, const OpArgs<R>* args,
-                                           const SignItem* signs, const PassParams<R>& P, uint64_t base) {
+// spread over the tile bits outside the cube).  FULL: every product formed (redo_tile).
+// With `last` it returns NaN when one of the thread's results is infinite or NaN.
+template <class R, bool FULL>
+__device__ __forceinline__ R tile_chain(uint32_t tile, uint32_t o, uint32_t gbase, const OpArgs<R>* args,
+                                           const SignItem* signs, const PassParams<R>& P, uint64_t base, bool last) {
   V<R>* const t = shared_tile<R>() + tile;  // an index into the shared array, so that accesses stay in the shared space
   const uint32_t nsub = P.head[o].em;
   const uint32_t cbits = P.head[o].gml;  // cube bit j: byte j
@@ -617,6 +619,35 @@ __device__ __forceinline__ void tile_chain(uint32_t tile, uint32_t o, uint32_t g
     const bool skip = (h.kind & DK_COND) && (base & P.cond[s].gfix) != P.cond[s].gval;  // uniform over the CTA
     const bool on = (gb & h.gml) == h.gvl;
     const uint32_t em = h.em;
+    uint32_t kind = skip ? 0u : h.kind & ~uint32_t(DK_COND);
+    if constexpr (FULL) {
+      const auto phase_on = [&](uint32_t elements, V<R> c) {
+#pragma unroll
+        for (int b = 0; b < CUBE; ++b)
+          if ((elements >> b) & 1) phase_in_place<R>(v[b], c);
+      };
+      if (kind >= DK_D1 && kind < DK_PH) {
+        kind = DK_D1 + (kind - DK_D1) % CUBE_BITS;
+      } else if (kind >= DK_TURN && kind <= DK_TURN_MASK) {
+        uint32_t half = 0;
+        for (uint32_t b = 0; b < CUBE; ++b)
+          if (kind == DK_TURN_ALL || ((b >> (kind - DK_TURN)) & 1)) half |= 1u << b;
+        V<R> c;
+        c.x = R(0);
+        c.y = op.a[0] ? R(1) : R(-1);
+        if (on) phase_on(kind == DK_TURN_MASK ? em : half, c);
+        continue;
+      } else if (kind == DK_SIGNS) {
+        V<R> c;
+        c.x = R(-1);
+        c.y = R(0);
+        for (uint32_t i = 0; i < em; ++i) {
+          const SignItem x = signs[h.gml + i];
+          if ((gb & x.fix) == x.fix && (base & x.gfix) == x.gfix) phase_on(x.em, c);
+        }
+        continue;
+      }
+    }
 #define NCSIM_D1(j) \
   case DK_D1 + j: chain_dense1<R, j>(v, op.c); break; \
   case DK_D1R + j: chain_dense1_real<R, j>(v, op.c); break; \
@@ -631,7 +662,7 @@ __device__ __forceinline__ void tile_chain(uint32_t tile, uint32_t o, uint32_t g
 #define NCSIM_SW(i, X) \
   case DK_SWAP + i: if (on) chain_swap<R, X>(v, em); break; \
   case DK_SWAPC + i: if (on) chain_swapc<R, X>(v, em & 0xffffu, em >> 16, op.c); break;
-    switch (skip ? 0u : h.kind & ~uint32_t(DK_COND)) {
+    switch (kind) {
       NCSIM_D1(0)
       NCSIM_D1(1)
       NCSIM_D1(2)
@@ -707,6 +738,38 @@ __device__ __forceinline__ void tile_chain(uint32_t tile, uint32_t o, uint32_t g
       if ((b >> j) & 1) a ^= sb[j];
     t[sg ^ a] = v[b];
   }
+  R odd = R(0);
+  if (last) {
+    R part[4] = {};  // short dependent chains
+#pragma unroll
+    for (int b = 0; b < CUBE; ++b) part[b & 3] = fma_rn(v[b].x, R(0), fma_rn(v[b].y, R(0), part[b & 3]));
+    odd = (part[0] + part[1]) + (part[2] + part[3]);
+  }
+  return odd;
+}
+
+// A tile whose amplitudes are not all finite, from the register again with every product formed: on an
+// infinite or NaN amplitude a product with zero is NaN, and the ops of the chains leave such products out.
+// (They keep what is not finite not finite, so the tile's results tell that one was met or made.)
+// The last chain's look at its results and a barrier that carries the answer cost 0.8% (n = 28) to 1.4% (n = 20) of
+// random layers; the same look in the op loop made its branches divergent ones (10%).
+template <class R>
+__device__ __noinline__ void redo_tile(uint32_t buf, uint64_t base, const OpArgs<R>* args, const SignItem* signs,
+                                       const uint16_t* cubes, uint64_t dthread, const uint64_t* dround, const PassParams<R>& P) {
+  const SwTile<R> t{shared_tile<R>() + buf};
+  for (uint32_t e = threadIdx.x, r = 0; e < 1u << P.g.T; e += blockDim.x, ++r) t[e] = P.amp[base | dthread | dround[r]];
+  __syncthreads();
+  for (uint32_t o = 0; o < P.nops; ++o) {
+    const OpHead& h = P.head[o];
+    if (h.kind == DK_CHAIN) {
+      tile_chain<R, true>(buf, o, cubes[h.gvl * blockDim.x + threadIdx.x], args, signs, P, base, false);
+      o += h.em;
+    } else {
+      if ((base & P.cond[o].gfix) != P.cond[o].gval) continue;
+      tile_sweep<R>(h.kind & ~uint32_t(DK_COND), buf, base, dthread, dround, args[o], P);
+    }
+    __syncthreads();
+  }
 }
 
 // One thread per cube of a tile: 2^(T - CUBE_BITS) threads, at least a warp, at most 128; the
@@ -776,17 +839,20 @@ __global__ void __launch_bounds__(3 * PASS_THREADS) k_plain_pass(const __grid_co
     }
     __syncthreads();
     const uint64_t base = tile_base_of(tile, g);
+    R odd = R(0);  // the last chain's
     for (uint32_t o = 0; o < P.nops; ++o) {
+      if (o) __syncthreads();
       const OpHead& h = P.head[o];
       if (h.kind == DK_CHAIN) {
-        tile_chain<R>(buf, o, cubes[h.gvl * blockDim.x + threadIdx.x], args, signs, P, base);
+        odd = tile_chain<R, false>(buf, o, cubes[h.gvl * blockDim.x + threadIdx.x], args, signs, P, base, h.gvl + 1 == P.nchains);
         o += h.em;
       } else {
         if ((base & P.cond[o].gfix) != P.cond[o].gval) continue;
         tile_sweep<R>(h.kind & ~uint32_t(DK_COND), buf, base, dthread, dround, args[o], P);
       }
-      __syncthreads();
     }
+    // outside the op loop, whose branches so stay uniform ones
+    if (__syncthreads_or(odd != odd)) redo_tile<R>(buf, base, args, signs, cubes, dthread, dround, P);
     V<R>* const dst = P.amp + (base | dthread);
     const V<R>* const from = shared_tile<R>() + buf;
     elements([&](uint32_t e, uint64_t off) { dst[off] = from[swz<R>(e)]; });
