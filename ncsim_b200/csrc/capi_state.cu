@@ -333,9 +333,11 @@ void state_sample(const ncsim_state* s, const double* uniforms, uint64_t shots, 
   NCSIM_CUDA(pool_alloc(&d.out, shots * sizeof(uint64_t), s->stream));
   NCSIM_CUDA(cudaMemcpyAsync(d.w, hi.data(), nblocks * sizeof(double), cudaMemcpyHostToDevice, s->stream));
   NCSIM_CUDA(cudaMemcpyAsync(d.u, uniforms, shots * sizeof(double), cudaMemcpyHostToDevice, s->stream));
-  // The parts read the register once more, a walk half a block per shot: they pay from about a shot
-  // per block on (1/128 of a complex128 register's bytes; without room for them the shots walk).
-  if (block == 4096 && shots >= nblocks) {
+  // The parts read the register once more, a walk half a block per shot: they pay from about a shot per
+  // block on, and from four shots (n = 12, one block: one shot 101 us with them and 84 without, two 101 and
+  // 93, four 100 and 102; 16384 shots 135 and 205).  1/256 of a complex128 register's bytes; without room for
+  // them the shots walk.
+  if (block == 4096 && shots >= std::max<uint64_t>(nblocks, 4)) {
     if (pool_alloc(&d.ends, nblocks * 32 * sizeof(double), s->stream) == cudaSuccess) {
       launch_sample_parts(s, d.w, nblocks, block, d.ends);
     } else {
