@@ -954,8 +954,8 @@ uint32_t cluster_size(const ncsim_batch* b, const ncsim_batch_config& cfg, const
   return best;
 }
 
-// one launch of the kernel over `count` jobs of the order array at order_off (`order`: those jobs, when
-// the launch may use clusters)
+// one launch of the kernel over `count` jobs of the order array at order_off (`order`, when the launch may
+// use clusters: the jobs that their size is chosen for, the whole batch's also where a sample of it is timed)
 void enqueue_kernel(ncsim_batch* b, const ncsim_batch_config& cfg, size_t order_off, uint32_t count,
                     const std::vector<uint32_t>* order) {
   check_launch_buffers(b);
@@ -1063,7 +1063,8 @@ ncsim_batch_config tune(ncsim_batch* b, uint32_t sample) {
                                b->stream));
     double ms = 1e300;
     for (int rep = 0; rep < 2; ++rep) {  // the first is a warm-up
-      enqueue_run(b, cf, b->off_sample, sample, false, true, &ord);
+      enqueue_run(b, cf, b->off_sample, sample, false, true,
+                  cf.order == NCSIM_BATCH_ORDER_GIVEN ? &b->order_seq : &b->order_lpt);
       const double t = finish_run(b);
       if (rep > 0) ms = std::min(ms, t);
     }
