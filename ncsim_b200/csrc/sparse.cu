@@ -1091,7 +1091,7 @@ ncsim_status ncsim_sparse_run(ncsim_sparse* s, const ncsim_circuit* c, ncsim_rng
     // reset or a gate that creates entries ends a run
     // one builder per host thread, reused so that its tables keep their capacity across runs
     static thread_local SlicedRun run;
-    run.reset();
+    run.release();
     std::vector<SparseDense1> dense;  // consecutive dense 1-qubit gates
     SparseDense1 d;
     for (const OpIR& op : c->ops) {
@@ -1119,6 +1119,7 @@ ncsim_status ncsim_sparse_run(ncsim_sparse* s, const ncsim_circuit* c, ncsim_rng
       if (r >= 0) rec[m++] = uint8_t(r);
     }
     run.launch(s);
+    run.release();
     sparse_apply_dense1(s, dense);
     NCSIM_CUDA(cudaStreamSynchronize(s->stream));
     if (len) *len = m;

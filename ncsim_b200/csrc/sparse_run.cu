@@ -20,6 +20,7 @@
 #include "sparse_run.hpp"
 
 #include <cstring>
+#include <type_traits>
 
 #include "sparse_common.cuh"
 
@@ -270,6 +271,20 @@ void SlicedRun::reset() {
   image_.clear();
   phase_.clear();
   unit_.clear();
+}
+
+void SlicedRun::release() {
+  reset();
+  const auto give_back = [](auto& v) {
+    if (v.capacity() * sizeof(v[0]) > KEPT_BYTES) std::remove_reference_t<decltype(v)>().swap(v);
+  };
+  give_back(stream_);
+  give_back(pending_);
+  give_back(image_);
+  give_back(phase_);
+  give_back(unit_);
+  blob_.clear();
+  give_back(blob_);
 }
 
 uint32_t* SlicedRun::put(uint32_t type, uint32_t words) {

@@ -18,6 +18,8 @@ class SlicedRun {
   bool empty() const { return !any_; }
   // empties the run; its buffers keep their capacity
   void reset();
+  // empties the run and gives buffers of more than KEPT_BYTES back: a host thread's run outlives its circuits
+  void release();
   // Adds a gate on the register's qubits; false when the gate creates entries or has no such form
   // (it then runs by itself).  `low` is the gate's lowering, on any qubit numbering.
   bool add_gate(const GateIR& g, const std::vector<uint32_t>& qubits, const LoweredOp& low);
@@ -27,6 +29,7 @@ class SlicedRun {
   void launch(ncsim_sparse* s);
 
  private:
+  static constexpr size_t KEPT_BYTES = size_t(1) << 20;
   struct Term {
     uint16_t q[3];
     uint8_t coeff;  // in 1/256 turns

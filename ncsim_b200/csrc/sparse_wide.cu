@@ -729,7 +729,7 @@ void sites_words(const PauliSites& ps, uint32_t words, std::vector<uint64_t>& x,
 template <int W>
 void run_w(ncsim_sparse* s, const ncsim_circuit& c, ncsim_rng& rng, uint8_t* rec, size_t& m) {
   static thread_local SlicedRun run;  // reused, so that its buffers keep their capacity
-  run.reset();
+  run.release();
   std::vector<uint64_t> x, z;
   std::vector<SparseDense1> dense;  // consecutive dense 1-qubit gates
   SparseDense1 d;
@@ -778,6 +778,7 @@ void run_w(ncsim_sparse* s, const ncsim_circuit& c, ncsim_rng& rng, uint8_t* rec
     }
   }
   run.launch(s);
+  run.release();
   sparse_apply_dense1(s, dense);
 }
 
