@@ -61,7 +61,7 @@ constexpr int GROUPS = 4;                                // four tiles in flight
 constexpr int COMPUTE_THREADS = GROUPS * GROUP_THREADS;  // warps 0-15
 constexpr int WARP_TILES = COMPUTE_THREADS / 32;         // warps 16-17: tile loads
 constexpr int TILE_THREADS = 64;
-constexpr int WARP_OPS = WARP_TILES + 2;                 // warp 18: B operand images and MMAs
+constexpr int WARP_OPS = WARP_TILES + 2;                 // warp 18: B operand images
 constexpr int WARP_FACTS = WARP_OPS + 1;                 // warp 19: what each tile's index bits decide
 constexpr int THREADS = COMPUTE_THREADS + TILE_THREADS + 64;
 constexpr int TILE = 1 << TILE_BITS;
@@ -309,7 +309,7 @@ __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
 }
 
 struct Tables : PassTables {
-  uint64_t bars[2 * NTILEBUF + 2 * NOPSLOT + 2 * GROUPS];  // tile full, tile done, operand full, operand empty, split, mma
+  uint64_t bars[2 * NTILEBUF + 2 * NOPSLOT + GROUPS];  // tile full, tile done, operand full, operand empty, mma
   float2 tab_lo[GROUPS][1 << HALF], tab_hi[GROUPS][1 << HALF];
   uint8_t tab_cross[GROUPS][1 << HALF];
   uint32_t act[NTILEBUF][MAX_CHUNKS];          // per tile: the chunks' terms active on it
@@ -438,8 +438,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused_pass(const __grid_constant
   auto bar_tdone = [&](uint32_t b) { return smem_u32(&S.bars[NTILEBUF + b]); };
   auto bar_ofull = [&](uint32_t s) { return smem_u32(&S.bars[2 * NTILEBUF + s]); };
   auto bar_oempty = [&](uint32_t s) { return smem_u32(&S.bars[2 * NTILEBUF + NOPSLOT + s]); };
-  auto bar_split = [&](int g) { return smem_u32(&S.bars[2 * NTILEBUF + 2 * NOPSLOT + g]); };
-  auto bar_mma = [&](int g) { return smem_u32(&S.bars[2 * NTILEBUF + 2 * NOPSLOT + GROUPS + g]); };
+  auto bar_mma = [&](int g) { return smem_u32(&S.bars[2 * NTILEBUF + 2 * NOPSLOT + g]); };
   auto fail = [&](int code) {
     S.abort = 1;
     atomicCAS(P.err, 0, code);
@@ -454,10 +453,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused_pass(const __grid_constant
       mbar_init(bar_ofull(i), 1);
       mbar_init(bar_oempty(i), NG);  // one commit (or release) per group
     }
-    for (int g = 0; g < GROUPS; ++g) {
-      mbar_init(bar_split(g), GROUP_THREADS / 32);
-      mbar_init(bar_mma(g), 1);
-    }
+    for (int g = 0; g < GROUPS; ++g) mbar_init(bar_mma(g), 1);
     S.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }

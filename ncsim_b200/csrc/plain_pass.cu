@@ -62,7 +62,7 @@ constexpr int MAX_PASS_OPS = 240;  // device ops of one pass (chain heads and fl
 constexpr int MAX_PASS_CHAINS = MAX_PASS_OPS / 3;
 // A chain's cube: CUBE_BITS tile bits, CUBE amplitudes held by one thread.  Four
 // bits: the op fetch and dispatch (about 25 instructions) are shared by 16
-// amplitudes, and a layer's 12 window qubits need 3 to 4 shared-memory round
+// amplitudes, and a layer's 11 window qubits need about 3 shared-memory round
 // trips.  The earlier three-bit cubes on 512 threads spent 54% of all issue slots
 // with the FP64 pipe 23% busy.
 constexpr int CUBE_BITS = 4;
@@ -1091,7 +1091,7 @@ struct PlainPlan {
   void* d_cpool = nullptr;
   uint32_t* d_upool = nullptr;
   uint64_t* d_ppool = nullptr;
-  size_t passes = 0, pass_gates = 0;
+  size_t passes = 0;
   ~PlainPlan() {
     if (device >= 0) {
       int cur = 0;
@@ -1466,7 +1466,6 @@ std::shared_ptr<PlainPlan> plan_plain_passes(uint32_t n, int precision, const st
       it.ops = chainify(ops, it.win.g.T, *P, it.signs);
       if (it.ops.size() > size_t(MAX_PASS_OPS)) throw Error(NCSIM_ERR_INVALID, "tiled pass: too many ops");
       P->passes += 1;
-      P->pass_gates += cur.size();
       P->items.push_back(std::move(it));
     }
     cur.clear();
