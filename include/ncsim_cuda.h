@@ -222,9 +222,10 @@ typedef struct ncsim_kernel_stat {
   double bytes;
 } ncsim_kernel_stat;
 /* Runs of 16 or more consecutive gates in ncsim_sv_run go through tiled passes
- * (on by default): a pass applies a run's gates to 4096-amplitude tiles in
+ * (on by default): a pass applies a run's gates to 2048-amplitude tiles in
  * shared memory, one HBM read and write for many gates, each gate with the
- * arithmetic of its own kernel (the amplitudes equal the gate-by-gate ones). */
+ * arithmetic of its own kernel (the amplitudes equal the gate-by-gate ones,
+ * infinite and NaN ones too). */
 ncsim_status ncsim_sv_set_tile_passes(ncsim_state* s, int32_t enable);
 ncsim_status ncsim_sv_profile_enable(ncsim_state* s, int32_t enable);
 ncsim_status ncsim_sv_profile_read(ncsim_state* s, ncsim_kernel_stat* out, uint32_t cap, uint32_t* count);
@@ -474,7 +475,9 @@ ncsim_status ncsim_sparse_tensor(const ncsim_sparse* a, const ncsim_sparse* b, n
 ncsim_status ncsim_sparse_sample(const ncsim_sparse* s, ncsim_rng* rng, uint64_t shots, uint64_t* out);
 /* to_vector (sparse.rs:426-434), n <= 26. */
 ncsim_status ncsim_sparse_to_vector(const ncsim_sparse* s, double* amps, uint64_t len);
-/* QuantumState::measure (mod.rs:113-131) and run (mod.rs:168-183) on the sparse state. */
+/* QuantumState::measure (mod.rs:113-131) and run (mod.rs:168-183) on the sparse state.  A run counts the
+ * phases of consecutive one-to-one gates and multiplies each amplitude by their product once, so its last
+ * bits (and, of an infinite or NaN amplitude, which parts are NaN) may differ from those of the gates one by one. */
 ncsim_status ncsim_sparse_measure(ncsim_sparse* s, uint64_t x, uint64_t z, uint32_t phase, ncsim_rng* rng,
                                   int32_t* outcome);
 ncsim_status ncsim_sparse_run(ncsim_sparse* s, const ncsim_circuit* c, ncsim_rng* rng, uint8_t* rec, size_t cap,
